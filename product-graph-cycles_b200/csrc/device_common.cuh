@@ -78,7 +78,9 @@ struct LiteralWalk {
 
 struct BfParams {
     // graph
-    int n, nY, K, Kp, nslices;
+    int n, nY, K, Kp, nslices, nslots;
+    const int* slotNode;           // [nslots] target node of a list slot (32 * slice + lane), -1: none
+    const int* nodeSlot;           // [n] slot of a node
     long long numNodes;            // n * nY
     const int* spInter;
     const int* spIntra;
@@ -100,6 +102,18 @@ struct BfParams {
     unsigned* stepDone;            // [ncta * kStepDoneStride] last step each CTA completed
     int flagSync;                  // 1: neighbour hand-offs between steps, 0: team barrier
     int maxCtaSlices;              // most slices any CTA owns
+    // sweeps on per-CTA local tables (bf_local.cuh): depths a table holds, 0
+    // when the sweeps work on the records in global memory
+    int localKD;
+    int localL, localHalo, localRows[2];  // most table entries, halo entries, rows per part of any CTA
+    int hopBits;                   // low bits of a packed (origin, length) word that hold the length
+    const unsigned short* lsrc[2]; // per list entry, its source's index in the owner CTA's table
+    const unsigned* haloSlot;      // [ncta * haloCap] halo slots of every CTA, ascending, with kHalo* bits
+    const int* haloCnt;            // [ncta]
+    int haloCap;
+    const unsigned* exposed;       // [nslices] lanes of a slice that another CTA reads
+    const unsigned char* sliceUsed;  // [nslices] the slice has rows or holds a source
+    uint4* xbuf;                   // [2][localKD][nslots] exchanged records
     int rowCap;                    // rows (of 32 entries) one step buffer holds
     int stageSrcOnly;              // 1: the buffers hold source indices only (costs, times prefetched to L2)
     int* lapNext;                  // [n]
@@ -206,6 +220,7 @@ constexpr long long kMedianCompact = 1 << 16;  // a bucket this small is selecte
 
 struct LookupArgs {
     int n, nY;
+    const int* nodeSlot;
     long long numNodes, eBlock;
     const int* spInter;
     const int* spIntra;
@@ -284,13 +299,14 @@ constexpr long long kWalkRoundLoads = 4096;
 constexpr int kBfThreads = 640;
 // Source values a lane gathers before folding them (one batch of rows).
 constexpr int kGather = 20;
-// Threads of a batched-solve CTA and the CTAs an SM should hold: each CTA
-// solves one graph at a time, so CTAs on one SM overlap their latencies.
-constexpr int kBatchThreads = 256;
+// Relaxing threads of a batched-solve CTA (one staging warp comes on top) and
+// the CTAs an SM holds: one, so that a graph's local tables and step buffers
+// get the SM's shared memory.
+constexpr int kBatchThreads = 640;
 // Capacity of a batched solve's cycle records (edges); a longer cycle hands
 // the graph back to the host.
 constexpr long long kBatchCycleCap = 1LL << 16;
-constexpr int kBatchBlocksPerSm = 2;
+constexpr int kBatchBlocksPerSm = 1;
 // Rows of one gather batch when every row has nk source depths (nk > 0).
 __host__ __device__ constexpr int bf_rows_per_batch(int nk) {
     return kGather / nk < 1 ? 1 : kGather / nk > 8 ? 8 : kGather / nk;
@@ -310,6 +326,51 @@ __host__ __device__ inline size_t bf_stage_offset(int maxCtaSlices) {
 __host__ __device__ inline size_t bf_stage_buffer_bytes(int rowCap, int costBytes, int timeBytes) {
     return (size_t)rowCap * 32 * (4 + costBytes + timeBytes);
 }
+// Byte offsets of a CTA's local tables in its dynamic shared memory (after
+// the step loop's parameters, bf_local.cuh); the step buffers follow at
+// `total`.
+constexpr size_t kLocalHotBytes = 384;
+struct LocalLayout {
+    size_t tslot, rec[2], gid, hslot, oh, val, lsrc[2], total;
+};
+__host__ __device__ inline LocalLayout local_layout(int maxSlices, int L, int halo, int rowsInter, int rowsIntra, int KD) {
+    LocalLayout o;
+    size_t at = kLocalHotBytes;
+    auto take = [&](size_t bytes) {
+        const size_t here = at;
+        at = (at + bytes + 15) & ~(size_t)15;
+        return here;
+    };
+    o.rec[0] = take((size_t)maxSlices * 16);
+    o.rec[1] = take((size_t)maxSlices * 16);
+    o.tslot = take((size_t)maxSlices * 2);
+    o.gid = take((size_t)L * 4);
+    o.hslot = take((size_t)halo * 4);
+    o.oh = take((size_t)2 * KD * L * 4);
+    o.val = take((size_t)2 * KD * L * 8);
+    o.lsrc[0] = take((size_t)rowsInter * 64);
+    o.lsrc[1] = take((size_t)rowsIntra * 64);
+    o.total = (at + 127) & ~(size_t)127;
+    return o;
+}
+// Most list slots the local plan's bitmaps hold in shared memory.
+constexpr int kLocalMaxSlots = 1 << 19;
+// The local tables' plan of a team (local_plan_kernel).
+struct LocalPlanArgs {
+    int nslices, ncta, parts;      // parts: 2 when the sweeps run intralayer steps
+    const int* ctaSlice;
+    const int* sp[2];
+    const int* src[2];
+    long long entries[2];
+    const int* nodeSlot;
+    unsigned char* used;
+    unsigned short* lsrc[2];
+    unsigned* haloSlot;
+    int haloCap;
+    int* counts;                   // [2][ncta] halo entries (may exceed haloCap: no plan), table slices
+    unsigned* exposed;
+};
+cudaError_t launch_local_plan(const LocalPlanArgs& a, int maxCtaSlices, cudaStream_t stream);
 // Attributes of a device that stay fixed while the process runs, queried
 // once per device (attribute queries can go to the driver and serialise
 // between host threads).
@@ -323,7 +384,8 @@ void note_launch();
 long long launch_count();
 cudaError_t launch_bf(const BfParams& p, int costIsF32, int timeKind, int blocks, int threads, bool cooperative,
                       bool sharedTables, size_t smemBytes, cudaStream_t stream);
-cudaError_t bf_max_coop_blocks(int costIsF32, int timeKind, int threads, size_t smemBytes, int* blocksPerSm);
+cudaError_t bf_max_coop_blocks(int costIsF32, int timeKind, bool local, int threads, size_t smemBytes,
+                               int* blocksPerSm);
 cudaError_t launch_extract_path(const BfParams& p, int v, cudaStream_t stream);
 // Batched ratio solves: `count` jobs taken from a queue (*next, zeroed by the
 // caller) by teams of `teamCtas` CTAs (blocks / teamCtas teams) of `threads`
@@ -372,11 +434,11 @@ cudaError_t launch_normals_3d(const double* V, long long nv, const int* F, long 
                               int* off, int* cursor, int* list, double* out, int* bad, cudaStream_t s);
 cudaError_t launch_normals_2d(const double* Vin, int nv, const int* E, double* V, double* en, double* el, double* out,
                               int* bad, cudaStream_t s);
-cudaError_t launch_layer1_mean(const double* cost, long long layerStride, long long interEntries, int n, int nslices,
-                               const int* spI, const int* spA, const int* srcI, const int* srcA, float* meanOut,
-                               int* countOut, cudaStream_t s);
-cudaError_t launch_layer1_mean(const float* cost, long long layerStride, long long interEntries, int n, int nslices,
-                               const int* spI, const int* spA, const int* srcI, const int* srcA, float* meanOut,
-                               int* countOut, cudaStream_t s);
+cudaError_t launch_layer1_mean(const double* cost, long long layerStride, long long interEntries, int n,
+                               const int* nodeSlot, const int* spI, const int* spA, const int* srcI, const int* srcA,
+                               float* meanOut, int* countOut, cudaStream_t s);
+cudaError_t launch_layer1_mean(const float* cost, long long layerStride, long long interEntries, int n,
+                               const int* nodeSlot, const int* spI, const int* spA, const int* srcI, const int* srcA,
+                               float* meanOut, int* countOut, cudaStream_t s);
 
 }  // namespace pgc

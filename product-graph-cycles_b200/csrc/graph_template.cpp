@@ -228,9 +228,73 @@ void build_conj(const int* EX, int64_t nEX, LayerTemplate& T) {
     });
 }
 
+// Slots in mesh order.  Vertices are ranked breadth first along the mesh
+// edges, so that consecutive ranks form a band of the mesh whose boundary is
+// short.  A plain node is a vertex; a conjugate node is an edge, ranked with
+// its tail, in one of three kinds whose in-degrees differ: 32 edges at a
+// time, a slice of each kind, so that a slice's nodes share their width and
+// a contiguous range of slices holds all kinds of its edges.
+void mesh_order(const int* EX, int64_t nEX, LayerTemplate& T) {
+    const int nv = T.conj ? T.nvx : T.n;
+    std::vector<int> ptr((size_t)nv + 1, 0), out((size_t)nEX), order;
+    for (int64_t e = 0; e < nEX; ++e) ++ptr[(size_t)EX[2 * e] + 1];
+    for (int v = 0; v < nv; ++v) ptr[(size_t)v + 1] += ptr[(size_t)v];
+    {
+        std::vector<int> fill(ptr.begin(), ptr.end() - 1);
+        for (int64_t e = 0; e < nEX; ++e) out[(size_t)fill[(size_t)EX[2 * e]]++] = (int)e;
+    }
+    order.reserve((size_t)nv);
+    std::vector<unsigned char> seen((size_t)nv, 0);
+    for (int r = 0; r < nv; ++r) {
+        if (seen[(size_t)r]) continue;
+        seen[(size_t)r] = 1;
+        size_t head = order.size();
+        order.push_back(r);
+        for (; head < order.size(); ++head) {
+            const int v = order[head];
+            for (int q = ptr[(size_t)v]; q < ptr[(size_t)v + 1]; ++q) {
+                const int w = EX[2 * out[(size_t)q] + 1];
+                if (seen[(size_t)w]) continue;
+                seen[(size_t)w] = 1;
+                order.push_back(w);
+            }
+        }
+    }
+    T.nodeSlot.resize((size_t)T.n);
+    if (!T.conj) {
+        T.nslices = (T.n + 31) / 32;
+        T.slotNode.resize((size_t)T.nslices * 32);
+        std::fill(T.slotNode.begin(), T.slotNode.end(), -1);
+        for (int i = 0; i < nv; ++i) {
+            T.slotNode[(size_t)i] = order[(size_t)i];
+            T.nodeSlot[(size_t)order[(size_t)i]] = i;
+        }
+        return;
+    }
+    T.nslices = 3 * (int)((nEX + 31) / 32);
+    T.slotNode.resize((size_t)T.nslices * 32);
+    std::fill(T.slotNode.begin(), T.slotNode.end(), -1);
+    int64_t rank = 0;
+    for (int v : order)
+        for (int q = ptr[(size_t)v]; q < ptr[(size_t)v + 1]; ++q, ++rank)
+            for (int kind = 0; kind < 3; ++kind) {
+                const int slot = (int)(((rank >> 5) * 3 + kind) * 32 + (rank & 31));
+                const int node = kind * (int)nEX + out[(size_t)q];
+                T.slotNode[(size_t)slot] = node;
+                T.nodeSlot[(size_t)node] = slot;
+            }
+}
+
 void build_sell(LayerTemplate& T) {
-    T.nslices = (T.n + 31) / 32;
+    if (T.slotNode.empty()) T.nslices = (T.n + 31) / 32;
     const int64_t n = T.n, nt = T.eBlock;
+    const int* slotNode = T.slotNode.empty() ? nullptr : T.slotNode.data();
+    // node of a list slot, or n where there is none
+    auto node_of = [=](int64_t slot) -> int64_t {
+        if (!slotNode) return slot;
+        const int v = slotNode[slot];
+        return v < 0 ? n : v;
+    };
     // In-edges of every (part, target) in ascending template edge id: one
     // stable counting sort on the key part * n + target, in parallel.  Chunk
     // c of the edge range counts its keys, the counts give each chunk its
@@ -291,7 +355,7 @@ void build_sell(LayerTemplate& T) {
         for (int s = 0; s < T.nslices; ++s) {
             int w = 0;
             for (int i = 0; i < 32; ++i) {
-                const int64_t v = 32LL * s + i;
+                const int64_t v = node_of(32LL * s + i);
                 if (v < n) w = std::max(w, pp[v + 1] - pp[v]);
             }
             sp[(size_t)s + 1] = sp[(size_t)s] + w;
@@ -311,7 +375,7 @@ void build_sell(LayerTemplate& T) {
             std::fill(T.src[p].begin() + r0, T.src[p].begin() + r1, -1);
             std::fill(T.tedge[p].begin() + r0, T.tedge[p].begin() + r1, -1);
             for (int i = 0; i < 32; ++i) {
-                const int64_t v = 32 * s + i;
+                const int64_t v = node_of(32 * s + i);
                 if (v >= n) continue;
                 for (int j = 0; j < pp[v + 1] - pp[v]; ++j) {
                     const int t = list[(size_t)(pp[v] + j)];
@@ -341,7 +405,7 @@ void host_parallel_for(int64_t n, int64_t grain, const std::function<void(int64_
 }
 
 std::string build_template(const int* EX, int64_t nEX, const int* EY, int64_t nEY, int64_t nVX, bool conj,
-                           bool prune, LayerTemplate& T) {
+                           bool prune, LayerTemplate& T, bool meshOrder) {
     if (nEX < 1) return "EX must have at least one row";
     if (nEY < 2) return "EY must have at least two rows (one product layer per Y edge)";
     int mx = -1;
@@ -367,6 +431,7 @@ std::string build_template(const int* EX, int64_t nEX, const int* EY, int64_t nE
         build_plain(EX, nEX, T);
     }
     T.eBlock = (int64_t)T.eSrc.size();
+    if (meshOrder) mesh_order(EX, nEX, T);
     build_sell(T);
     (void)EY;
     return "";
@@ -495,6 +560,46 @@ std::vector<int> plan_cta_cuts(const LayerTemplate& T, int blocks, int K, int wa
     return cut;
 }
 
+// A slice's work in one layer: per row its entry's loads and weight, then a
+// sum and a comparison per source depth, plus the epilogue of every step that
+// visits it (issue slots, roughly).
+std::vector<int> plan_even_cuts(const LayerTemplate& T, int blocks, int K) {
+    const int ns = T.nslices;
+    std::vector<int> cut((size_t)blocks + 1, ns);
+    cut[0] = 0;
+    if (blocks <= 1 || ns == 0) return cut;
+    const int reps = T.entries[INTRA] > 0 ? K - 1 : 0, nk = reps > 0 ? K : 1;
+    std::vector<long long> acc((size_t)ns + 1, 0);
+    long long top = 0;
+    for (int s = 0; s < ns; ++s) {
+        const int ri = T.sp[INTER][(size_t)s + 1] - T.sp[INTER][(size_t)s];
+        const int ra = reps ? T.sp[INTRA][(size_t)s + 1] - T.sp[INTRA][(size_t)s] : 0;
+        const long long w = (ri ? 30 + ri * (9LL + 6 * nk) : 0) + (ra ? reps * (30 + ra * 15LL) : 0) + 1;
+        acc[(size_t)s + 1] = acc[(size_t)s] + w;
+        top = std::max(top, w);
+    }
+    // the smallest bound on a range's work that `blocks` ranges satisfy
+    auto fill = [&](long long bound, std::vector<int>* c) {
+        int used = 0, s = 0;
+        while (s < ns) {
+            const long long end = acc[(size_t)s] + bound;
+            s = (int)(std::upper_bound(acc.begin() + s + 1, acc.end(), end) - acc.begin()) - 1;
+            if (++used > blocks) return used;
+            if (c) (*c)[(size_t)used] = s;
+        }
+        return used;
+    };
+    long long lo = std::max(top, (acc[(size_t)ns] + blocks - 1) / blocks), hi = acc[(size_t)ns];
+    while (lo < hi) {
+        const long long mid = lo + (hi - lo) / 2;
+        if (fill(mid, nullptr) <= blocks) hi = mid;
+        else lo = mid + 1;
+    }
+    const int used = fill(lo, &cut);
+    for (int c = used + 1; c <= blocks; ++c) cut[(size_t)c] = ns;
+    return cut;
+}
+
 // Wait lists of the Bellman-Ford team in CSR form (ptr: blocks + 1 offsets,
 // idx: CTA ids, ascending per list): CTA c lists every other CTA d joined to
 // it by an in-edge of either part, i.e. d owns the slice of a source of one
@@ -522,7 +627,7 @@ void cta_wait_lists(const LayerTemplate& T, const std::vector<int>& cut, std::ve
                     for (int lane = 0; lane < 32; ++lane) {
                         const int sv = T.src[p][(size_t)j * 32 + lane];
                         if (sv < 0) continue;
-                        const int cs = owner[(size_t)(sv >> 5)];
+                        const int cs = owner[(size_t)((T.nodeSlot.empty() ? sv : T.nodeSlot[(size_t)sv]) >> 5)];
                         if (cs == ct || cs == last) continue;
                         last = cs;
                         mine[(size_t)ct * blocks + cs] = 1;

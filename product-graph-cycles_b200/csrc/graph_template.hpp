@@ -88,6 +88,9 @@ struct LayerTemplate {
     RawVec<int> sp[2];             // nslices + 1 slot offsets
     RawVec<int> src[2];            // 32 * slots: local source node or -1
     RawVec<int> tedge[2];          // 32 * slots: template edge offset or -1
+    // Target node of every list slot (32 * slice + lane; -1: no node) and the
+    // slot of every node.  Empty: node v has slot v.
+    RawVec<int> slotNode, nodeSlot;
     RawVec<int> srcDummy;          // INTER src list of the closing layer; stored for nY == 2 only (else == src[INTER])
     int64_t entries[2] = {0, 0};   // 32 * slots per part
     // per template edge offset (eBlock entries)
@@ -102,8 +105,10 @@ struct LayerTemplate {
 };
 
 // Builds the template; returns an empty string or an error message.
+// meshOrder: the list slots follow the mesh (slotNode, nodeSlot) instead of
+// the node ids, so that a contiguous range of slices is a patch of it.
 std::string build_template(const int* EX, int64_t nEX, const int* EY, int64_t nEY, int64_t nVX, bool conj,
-                           bool prune, LayerTemplate& T);
+                           bool prune, LayerTemplate& T, bool meshOrder = false);
 
 // Runs f(begin, end) over parts of [0, n) of at least `grain` items on the
 // process's host worker pool (inline when another job holds the pool).
@@ -113,6 +118,11 @@ void host_parallel_for(int64_t n, int64_t grain, const std::function<void(int64_
 // warps for the Bellman-Ford team, balanced on the per-step work of their
 // slowest warps; rowsPerBatch[p] = rows a warp gathers per batch in part p.
 std::vector<int> plan_cta_cuts(const LayerTemplate& T, int blocks, int K, int warps, const int rowsPerBatch[2]);
+
+// Contiguous slice ranges of `blocks` CTAs balanced on the summed work of
+// their slices: the ranges of teams that keep their nodes' values on chip,
+// where a CTA's step time follows its issue slots, not its slowest warp.
+std::vector<int> plan_even_cuts(const LayerTemplate& T, int blocks, int K);
 
 // Wait lists of the Bellman-Ford team for the CTA slice ranges `cut`: CTA c
 // lists, in ascending order in idx[ptr[c]..ptr[c+1]), every other CTA joined

@@ -17,13 +17,12 @@
 //  * predecessors are written only on improvement, so stale entries evolve as
 //    in the reference.
 //
-// Work split of one (layer, depth) step: every CTA owns a range of node
-// slices (32 nodes each) balanced by in-edge entries.  Phase A: the CTA's
-// threads take the in-edge entries of a chunk of slices independently --
-// source index, cost and time, then the source's DP record -- and leave each
-// entry's best candidate in shared memory, so a whole chunk costs two memory
-// latencies however large the in-degree.  Phase B: one thread per node folds
-// its entries in edge order (the reference's tie-break) and writes the node.
+// Work split of one (layer, depth) step: every CTA owns a range of slices of
+// 32 list slots; a warp relaxes a slice, one lane per target node, its rows in
+// edge order (the reference's tie-break).  Teams that can keep the DP records
+// they need in shared memory (bf_local.cuh), which is every graph of up to
+// four depths whose tables fit; the others gather the sources from global
+// memory and hand steps off through per-CTA counters.
 //
 // Cycle detection: the reference walks predecessors from every negative
 // start node in ascending order of its value until a start node repeats.
@@ -398,11 +397,7 @@ __device__ __forceinline__ double edge_weight(const StepView& v, int q) {
 // One batch of exactly NR rows starting at `row`: every source value is
 // gathered first, then the batch is folded in edge order.  `win` records the
 // position of the last improvement (row * 8 + depth); thr is its value.
-// TREE: the batch's candidates are reduced as a balanced tree of (value,
-// position) minima instead of one sequential compare chain (the batched
-// kernel, whose register budget holds the extra live values; the
-// single-graph kernel's 96-register budget does not).
-template <class CT, int TK, bool S, int NK, int NR, bool TREE>
+template <class CT, int TK, bool S, int NK, int NR>
 __device__ __forceinline__ void fold_batch(const StepView& v, int lane, int row, double& thr, int& win) {
     int sv[NR];
     double d[NR][NK];
@@ -416,53 +411,14 @@ __device__ __forceinline__ void fold_batch(const StepView& v, int lane, int row,
             for (int kk = 0; kk < NK; ++kk) d[r][kk] = kInfD;
         }
     }
-    if constexpr (!TREE) {
 #pragma unroll
-        for (int r = 0; r < NR; ++r) {
-            if (sv[r] < 0) continue;
-            const double w = edge_weight<CT, TK>(v, (row + r) * 32 + lane);
+    for (int r = 0; r < NR; ++r) {
+        if (sv[r] < 0) continue;
+        const double w = edge_weight<CT, TK>(v, (row + r) * 32 + lane);
 #pragma unroll
-            for (int kk = 0; kk < NK; ++kk) {
-                const double cand = __dadd_rn(d[r][kk], w);
-                if (cand < thr) { thr = cand; win = ((row + r) << 3) | kk; }
-            }
-        }
-    } else {
-        // The candidates in edge order (row, then depth), reduced so that
-        // the left -- earlier -- candidate wins ties: the first minimum,
-        // which is what the sequential scan `cand < thr` ends with.  A NaN
-        // candidate, which that scan never takes, enters as +inf; neither
-        // is ever below thr.
-        constexpr int N = NR * NK;
-        double cv[N];
-        int ci[N];
-#pragma unroll
-        for (int r = 0; r < NR; ++r) {
-            const double w = sv[r] >= 0 ? edge_weight<CT, TK>(v, (row + r) * 32 + lane) : 0.0;
-#pragma unroll
-            for (int kk = 0; kk < NK; ++kk) {
-                double c = kInfD;
-                if (sv[r] >= 0) {
-                    c = __dadd_rn(d[r][kk], w);
-                    if (c != c) c = kInfD;
-                }
-                cv[r * NK + kk] = c;
-                ci[r * NK + kk] = r * NK + kk;
-            }
-        }
-#pragma unroll
-        for (int s = 1; s < N; s <<= 1) {
-#pragma unroll
-            for (int i = 0; i + s < N; i += 2 * s) {
-                if (cv[i + s] < cv[i]) {
-                    cv[i] = cv[i + s];
-                    ci[i] = ci[i + s];
-                }
-            }
-        }
-        if (cv[0] < thr) {
-            thr = cv[0];
-            win = ((row + ci[0] / NK) << 3) | (ci[0] % NK);
+        for (int kk = 0; kk < NK; ++kk) {
+            const double cand = __dadd_rn(d[r][kk], w);
+            if (cand < thr) { thr = cand; win = ((row + r) << 3) | kk; }
         }
     }
 }
@@ -470,26 +426,26 @@ __device__ __forceinline__ void fold_batch(const StepView& v, int lane, int row,
 // The last nr (1 <= nr <= NR) rows as one batch of exactly nr rows.  The row
 // count is the slice's, the same in every lane, so no lane runs row slots
 // that do not exist.
-template <class CT, int TK, bool S, int NK, int NR, bool TREE>
+template <class CT, int TK, bool S, int NK, int NR>
 __device__ __forceinline__ void fold_tail(const StepView& v, int lane, int row, int nr, double& thr, int& win) {
     if constexpr (NR <= 1) {
-        fold_batch<CT, TK, S, NK, 1, TREE>(v, lane, row, thr, win);
+        fold_batch<CT, TK, S, NK, 1>(v, lane, row, thr, win);
     } else {
-        if (nr == NR) fold_batch<CT, TK, S, NK, NR, TREE>(v, lane, row, thr, win);
-        else fold_tail<CT, TK, S, NK, NR - 1, TREE>(v, lane, row, nr, thr, win);
+        if (nr == NR) fold_batch<CT, TK, S, NK, NR>(v, lane, row, thr, win);
+        else fold_tail<CT, TK, S, NK, NR - 1>(v, lane, row, nr, thr, win);
     }
 }
 
 // Rows [row, j1) of one slice for lane `lane`.  Returns the position of the
 // winning candidate -- row * 8 + depth for NK > 0, row * nk + depth for the
 // run-time depth count (NK == 0) -- or -1; thr holds its value.
-template <class CT, int TK, bool S, int NK, bool TREE>
+template <class CT, int TK, bool S, int NK>
 __device__ __forceinline__ int fold_rows(const StepView& v, int lane, int row, int j1, double& thr) {
     int win = -1;
     if constexpr (NK > 0) {
         constexpr int RB = bf_rows_per_batch(NK);
-        for (; j1 - row >= RB; row += RB) fold_batch<CT, TK, S, NK, RB, TREE>(v, lane, row, thr, win);
-        if (row < j1) fold_tail<CT, TK, S, NK, RB, TREE>(v, lane, row, j1 - row, thr, win);
+        for (; j1 - row >= RB; row += RB) fold_batch<CT, TK, S, NK, RB>(v, lane, row, thr, win);
+        if (row < j1) fold_tail<CT, TK, S, NK, RB>(v, lane, row, j1 - row, thr, win);
     } else {
         for (; row < j1; ++row) {
             const int sv = v.src[row * 32 + lane];
@@ -505,7 +461,7 @@ __device__ __forceinline__ int fold_rows(const StepView& v, int lane, int row, i
     return win;
 }
 
-template <class CT, int TK, bool S, int NK, bool TREE>
+template <class CT, int TK, bool S, int NK>
 __device__ bool relax_slices(const BfParams& p, const StepView& sv, const int* spl, const int* act, int nAct, int s0,
                              int s1, int l, int k) {
     const int n = p.n, K = p.K, Kp = p.Kp;
@@ -529,13 +485,13 @@ __device__ bool relax_slices(const BfParams& p, const StepView& sv, const int* s
     const int count = all ? s1 - s0 : nAct;
     for (int i = (int)(threadIdx.x >> 5); i < count; i += nwarps) {
         const int s = s0 + (all ? i : act[i]);
-        const int v = s * 32 + lane;
-        const bool valid = v < n;
+        const int v = __ldg(p.slotNode + s * 32 + lane);
+        const bool valid = v >= 0;
         const size_t me = cur + (size_t)v * Kp + k;
         double best = (l == 0 && valid) ? ldV<S>(p, me) : kInfD;
         double thr = best < ub ? best : ub;
         int win = -1;
-        if (!empty) win = fold_rows<CT, TK, S, NK, TREE>(sv, lane, spl[s - s0] - r0, spl[s + 1 - s0] - r0, thr);
+        if (!empty) win = fold_rows<CT, TK, S, NK>(sv, lane, spl[s - s0] - r0, spl[s + 1 - s0] - r0, thr);
         if (!valid) continue;
         int o = kLapUnknown, h = 0;
         int bs = -1, bk = -1;
@@ -580,7 +536,7 @@ __device__ bool relax_slices(const BfParams& p, const StepView& sv, const int* s
     return any;
 }
 
-template <class CT, int TK, bool S, bool TREE>
+template <class CT, int TK, bool S>
 __device__ bool relax_step(const BfParams& p, const Stage& st, int sb, int s0, int s1, int l, int k) {
     const int n = p.n, K = p.K, Kp = p.Kp;
     const bool inter = (k == 0);
@@ -612,13 +568,13 @@ __device__ bool relax_step(const BfParams& p, const Stage& st, int sb, int s0, i
     v.tconst = p.tconst;
     const int* act = st.act(part);
     const int na = st.nAct(part);
-    if (!inter) return relax_slices<CT, TK, S, 1, TREE>(p, v, spl, act, na, s0, s1, l, k);
+    if (!inter) return relax_slices<CT, TK, S, 1>(p, v, spl, act, na, s0, s1, l, k);
     switch (K) {
-        case 1: return relax_slices<CT, TK, S, 1, TREE>(p, v, spl, act, na, s0, s1, l, k);
-        case 2: return relax_slices<CT, TK, S, 2, TREE>(p, v, spl, act, na, s0, s1, l, k);
-        case 3: return relax_slices<CT, TK, S, 3, TREE>(p, v, spl, act, na, s0, s1, l, k);
-        case 4: return relax_slices<CT, TK, S, 4, TREE>(p, v, spl, act, na, s0, s1, l, k);
-        default: return relax_slices<CT, TK, S, 0, TREE>(p, v, spl, act, na, s0, s1, l, k);
+        case 1: return relax_slices<CT, TK, S, 1>(p, v, spl, act, na, s0, s1, l, k);
+        case 2: return relax_slices<CT, TK, S, 2>(p, v, spl, act, na, s0, s1, l, k);
+        case 3: return relax_slices<CT, TK, S, 3>(p, v, spl, act, na, s0, s1, l, k);
+        case 4: return relax_slices<CT, TK, S, 4>(p, v, spl, act, na, s0, s1, l, k);
+        default: return relax_slices<CT, TK, S, 0>(p, v, spl, act, na, s0, s1, l, k);
     }
 }
 
@@ -663,6 +619,8 @@ __device__ bool step_handoff(const BfParams& p, const Team& t, unsigned step) {
     __syncthreads();
     return *(volatile int*)t.err == 0;
 }
+
+#include "bf_local.cuh"
 
 // Brent's cycle finding on the lap function starting at x0.
 // Returns 1 (cycle: first repeated node in *v0, steps in *steps),
@@ -915,8 +873,12 @@ __device__ int dij_walk_end(const BfParams& p, int v) {
 // the dynamic shared memory after the DP tables: [row offsets and lists of
 // slices with rows][two step buffers].
 // ---------------------------------------------------------------------------
-template <class CT, int TK, bool S, bool TREE = false>
+// SITE > 0: the sweeps run on per-CTA local tables (bf_local.cuh), which take
+// all of the dynamic shared memory; the number keeps the kernels' instances of
+// the step loop apart.
+template <class CT, int TK, bool S, int SITE = 0>
 __device__ __forceinline__ void bf_body(const BfParams& p, const Team& t, char* smem) {
+    constexpr bool LOCAL = SITE > 0;
     const int n = p.n, K = p.K, Kp = p.Kp;
     const long long tid = t.thread(), nth = t.nthreads();
     const bool isLead = (t.cta == 0 && threadIdx.x == 0);
@@ -928,7 +890,7 @@ __device__ __forceinline__ void bf_body(const BfParams& p, const Team& t, char* 
     __shared__ unsigned long long stageBar[2];
     __shared__ int nActive[2];
     Stage st;
-    {
+    if constexpr (!LOCAL) {
         int* spl0 = reinterpret_cast<int*>(smem);
         int* spl1 = spl0 + p.maxCtaSlices + 1;
         int* act0 = spl1 + p.maxCtaSlices + 1;
@@ -981,6 +943,13 @@ __device__ __forceinline__ void bf_body(const BfParams& p, const Team& t, char* 
         st.nActIntra = nActive[1];
     }
 
+    unsigned phase = 0;
+    if constexpr (LOCAL) {
+        local_begin(p, t, s0, s1, sizeof(CT), TK == 1 ? 4 : TK == 2 ? 8 : 0);
+        // no record carries a step number yet
+        if (t.ncta > 1)
+            for (long long r = tid; r < 2LL * p.localKD * p.nslots; r += nth) p.xbuf[r] = make_uint4(0, 0, 0, 0);
+    }
     // set-up (cost_time_ratio_solver.cpp:264-287): DP := inf, branch starts := 0
     // (each record is written once, by one thread)
     for (long long r = tid; r < 2LL * n * Kp; r += nth) {
@@ -1040,10 +1009,15 @@ __device__ __forceinline__ void bf_body(const BfParams& p, const Team& t, char* 
     // interlayer step of each layer runs.
     const int kSteps = p.intraEntries == 0 ? 1 : K;
     for (;;) {
-        // the first step of the sweep is staged while the backup row is copied
-        stage_issue(p, st, s0, s1, 0, kSteps > 1 ? 0 : 1, kSteps > 1 ? 1 : 0);
+        if constexpr (!LOCAL) {
+            // the first step of the sweep is staged while the backup row is copied
+            stage_issue(p, st, s0, s1, 0, kSteps > 1 ? 0 : 1, kSteps > 1 ? 1 : 0);
+        }
         for (long long i = tid; i < n; i += nth) p.bak[i] = ldV<S>(p, (size_t)i * Kp);
-        if (!team_sync(t)) { stage_drain(st); return; }
+        if (!team_sync(t)) {
+            if constexpr (!LOCAL) stage_drain(st);
+            return;
+        }
         // Layers are relaxed in order; a CTA hands each step off to its
         // graph neighbours only (one team barrier closes the sweep).  The
         // reference stops a sweep at the first layer 1..nY-1 without an
@@ -1053,38 +1027,61 @@ __device__ __forceinline__ void bf_body(const BfParams& p, const Team& t, char* 
         const int stamp = epochBase + sweep + 1;
         const unsigned long long tRelax = isLead ? clock64() : 0;
         unsigned long long cycRelax = 0, cycHand = 0, cycStage = 0;
-        int sb = 0;  // buffer of the current step
-        for (int l = 0; l <= p.nY; ++l) {
-            for (int k = 0; k < kSteps; ++k) {
-                if (l == 0 && k == 0) continue;
-                const unsigned long long ta = isLead ? clock64() : 0;
-                if (!stage_wait(st, sb)) {
-                    atomicExch(t.err, 1);
-                    stage_drain(st);
-                    return;
-                }
-                if (isLead) cycStage += clock64() - ta;
-                const bool last = l == p.nY && k == kSteps - 1;
-                if (!last) stage_issue(p, st, s0, s1, sb ^ 1, k + 1 < kSteps ? l : l + 1, k + 1 < kSteps ? k + 1 : 0);
-                const bool any = relax_step<CT, TK, S, TREE>(p, st, sb, s0, s1, l, k);
-                if (__any_sync(0xffffffffu, any) && (threadIdx.x & 31) == 0) p.layerFlag[l] = stamp;
-                const unsigned long long tb = isLead ? clock64() : 0;
-                ++step;
-                sb ^= 1;
-                const bool ok = (handoff && !last) ? step_handoff(p, t, step) : team_sync(t);
-                if (!ok) {
-                    stage_drain(st);
-                    return;
-                }
-                if (isLead) {
-                    const unsigned long long tc = clock64();
-                    cycRelax += tb - ta;
-                    cycHand += tc - tb;
+        if constexpr (LOCAL) {
+            LocalHot& H = local_hot();
+            if (isLead) H.cyc[0] = H.cyc[1] = H.cyc[2] = 0;
+            local_load(p);
+            __syncthreads();
+            switch (p.localKD) {
+                case 1: phase = local_sweep<CT, TK, 1, SITE>(stamp, step, phase); break;
+                case 2: phase = local_sweep<CT, TK, 2, SITE>(stamp, step, phase); break;
+                case 3: phase = local_sweep<CT, TK, 3, SITE>(stamp, step, phase); break;
+                default: phase = local_sweep<CT, TK, 4, SITE>(stamp, step, phase); break;
+            }
+            if (phase & 4u) {
+                atomicExch(t.err, 1);
+                return;
+            }
+            step += (unsigned)(p.nY * p.localKD);
+            local_store(p);
+            cycRelax = H.cyc[0];
+            cycHand = H.cyc[1];
+            cycStage = H.cyc[2];
+            if (!team_sync(t)) return;
+        } else {
+            int sb = 0;  // buffer of the current step
+            for (int l = 0; l <= p.nY; ++l) {
+                for (int k = 0; k < kSteps; ++k) {
+                    if (l == 0 && k == 0) continue;
+                    const unsigned long long ta = isLead ? clock64() : 0;
+                    if (!stage_wait(st, sb)) {
+                        atomicExch(t.err, 1);
+                        stage_drain(st);
+                        return;
+                    }
+                    if (isLead) cycStage += clock64() - ta;
+                    const bool last = l == p.nY && k == kSteps - 1;
+                    if (!last) stage_issue(p, st, s0, s1, sb ^ 1, k + 1 < kSteps ? l : l + 1, k + 1 < kSteps ? k + 1 : 0);
+                    const bool any = relax_step<CT, TK, S>(p, st, sb, s0, s1, l, k);
+                    if (__any_sync(0xffffffffu, any) && (threadIdx.x & 31) == 0) p.layerFlag[l] = stamp;
+                    const unsigned long long tb = isLead ? clock64() : 0;
+                    ++step;
+                    sb ^= 1;
+                    const bool ok = (handoff && !last) ? step_handoff(p, t, step) : team_sync(t);
+                    if (!ok) {
+                        stage_drain(st);
+                        return;
+                    }
+                    if (isLead) {
+                        const unsigned long long tc = clock64();
+                        cycRelax += tb - ta;
+                        cycHand += tc - tb;
+                    }
                 }
             }
         }
         int stopHere = 0;
-        for (int l = 1 + (int)threadIdx.x; l < p.nY; l += blockDim.x)
+        for (int l = (LOCAL ? p.nY - 1 : 1) + (int)threadIdx.x; l < p.nY; l += blockDim.x)
             if (*(volatile int*)(p.layerFlag + l) != stamp) stopHere = 1;
         const bool stop = __syncthreads_or(stopHere) != 0;
         ++sweep;
@@ -1389,7 +1386,6 @@ __device__ __forceinline__ void bf_body(const BfParams& p, const Team& t, char* 
 template <class CT, int TK, bool S>
 __global__ void __launch_bounds__(kBfThreads, 1) bf_kernel(BfParams p) {
     const Team t{(int)blockIdx.x, (int)gridDim.x, &p.ctl->barCount, &p.ctl->barGen, &p.ctl->error, p.spinLimit};
-    extern __shared__ double4 smemRaw[];
     char* smem = reinterpret_cast<char*>(smemRaw);
     if constexpr (S) {
         // single-CTA team: the DP records and the backup row live in shared
@@ -1400,6 +1396,104 @@ __global__ void __launch_bounds__(kBfThreads, 1) bf_kernel(BfParams p) {
         smem += bf_shared_table_bytes(p.n, p.Kp);
     }
     bf_body<CT, TK, S>(p, t, smem);
+}
+
+// The same on per-CTA local tables (bf_local.cuh).
+template <class CT, int TK>
+__global__ void __launch_bounds__(kBfThreads + 32, 1) bf_local_kernel(const __grid_constant__ BfParams p) {
+    const Team t{(int)blockIdx.x, (int)gridDim.x, &p.ctl->barCount, &p.ctl->barGen, &p.ctl->error, p.spinLimit};
+    bf_body<CT, TK, false, 1>(p, t, nullptr);
+}
+
+// Which list entry reads which entry of its CTA's local table.  First the
+// slices that need table entries: those with rows, and those with a source.
+__global__ void local_used_kernel(LocalPlanArgs a) {
+    const long long nth = (long long)gridDim.x * blockDim.x, tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    for (int part = 0; part < 2; ++part) {
+        for (long long s = tid; s < a.nslices; s += nth)
+            if (a.sp[part][s + 1] > a.sp[part][s]) a.used[s] = 1;
+        for (long long e = tid; e < a.entries[part]; e += nth) {
+            const int v = a.src[part][e];
+            if (v >= 0) a.used[a.nodeSlot[v] >> 5] = 1;
+        }
+    }
+}
+
+// Then, one CTA per CTA of the team: a bitmap over all slots of the sources
+// outside its slices (one word per slice), their ranks by prefix sum -- the
+// halo in ascending slot order -- and every entry's local index.
+__global__ void local_plan_kernel(LocalPlanArgs a) {
+    extern __shared__ unsigned planSh[];
+    unsigned* bits = planSh;                    // [nslices]
+    unsigned* pre = planSh + a.nslices;         // [nslices] halo entries before the slice
+    unsigned* tab = planSh + 2 * a.nslices;     // [own slices] table slice
+    __shared__ unsigned part512[512];
+    __shared__ unsigned total, tables;
+    const int c = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
+    const int s0 = a.ctaSlice[c], s1 = a.ctaSlice[c + 1];
+    for (int i = tid; i < a.nslices; i += nt) bits[i] = 0;
+    __syncthreads();
+    for (int part = 0; part < a.parts; ++part) {
+        const long long e0 = (long long)a.sp[part][s0] * 32, e1 = (long long)a.sp[part][s1] * 32;
+        for (long long e = e0 + tid; e < e1; e += nt) {
+            const int v = a.src[part][e];
+            if (v < 0) continue;
+            const int slot = a.nodeSlot[v], sl = slot >> 5;
+            if (sl < s0 || sl >= s1) atomicOr(bits + sl, 1u << (slot & 31));
+        }
+    }
+    __syncthreads();
+    // exclusive prefix sums: halo entries per slice, then used own slices
+    auto scan = [&](int n, auto count, unsigned* out, unsigned* sum) {
+        const int per = (n + nt - 1) / nt, b0 = min(tid * per, n), b1 = min(b0 + per, n);
+        unsigned mine = 0;
+        for (int i = b0; i < b1; ++i) mine += count(i);
+        part512[tid] = mine;
+        __syncthreads();
+        for (int o = 1; o < nt; o <<= 1) {
+            const unsigned x = tid >= o ? part512[tid - o] : 0;
+            __syncthreads();
+            part512[tid] += x;
+            __syncthreads();
+        }
+        unsigned at = tid ? part512[tid - 1] : 0;
+        for (int i = b0; i < b1; ++i) {
+            out[i] = at;
+            at += count(i);
+        }
+        if (tid == nt - 1) *sum = part512[tid];
+        __syncthreads();
+    };
+    scan(a.nslices, [&](int i) { return (unsigned)__popc(bits[i]); }, pre, &total);
+    scan(s1 - s0, [&](int i) { return a.used[s0 + i] ? 1u : 0u; }, tab, &tables);
+    const unsigned nHalo = total, nOwn = 32 * tables;
+    if (tid == 0) {
+        a.counts[c] = (int)nHalo;
+        a.counts[a.ncta + c] = (int)tables;
+    }
+    if (nHalo > (unsigned)a.haloCap || nOwn + nHalo + 1 > 0xffffu) return;  // the host sees the counts
+    for (int i = tid; i < a.nslices; i += nt) {
+        unsigned m = bits[i];
+        if (!m) continue;
+        atomicOr(a.exposed + i, m);
+        const unsigned rows = (a.sp[0][i + 1] > a.sp[0][i] ? kHaloInter : 0u) |
+                              (a.parts > 1 && a.sp[1][i + 1] > a.sp[1][i] ? kHaloIntra : 0u);
+        unsigned* out = a.haloSlot + (size_t)c * a.haloCap + pre[i];
+        for (; m; m &= m - 1) *out++ = (unsigned)(i * 32 + __ffs(m) - 1) | rows;
+    }
+    for (int part = 0; part < a.parts; ++part) {
+        const long long e0 = (long long)a.sp[part][s0] * 32, e1 = (long long)a.sp[part][s1] * 32;
+        for (long long e = e0 + tid; e < e1; e += nt) {
+            const int v = a.src[part][e];
+            unsigned at = nOwn + nHalo;  // an empty slot's source: the +inf entry
+            if (v >= 0) {
+                const int slot = a.nodeSlot[v], sl = slot >> 5, lane = slot & 31;
+                if (sl >= s0 && sl < s1) at = tab[sl - s0] * 32 + lane;
+                else at = nOwn + pre[sl] + __popc(bits[sl] & ((1u << lane) - 1u));
+            }
+            a.lsrc[part][e] = (unsigned short)at;
+        }
+    }
 }
 
 // Minimum-cost path extraction (dijkstra_solver.cpp:349-357): from the
@@ -1449,7 +1543,7 @@ __device__ bool lookup_edge(const LookupArgs& a, long long S, long long T, long 
     } else {
         return false;
     }
-    const int slice = v >> 5, lane = v & 31;
+    const int slot = a.nodeSlot[v], slice = slot >> 5, lane = slot & 31;
     for (int j = sp[slice]; j < sp[slice + 1]; ++j) {
         const long long e = (long long)j * 32 + lane;
         if (src[e] == s) {
@@ -1568,21 +1662,28 @@ __device__ int record_cycle(const PairJob& J, const BfParams& P, const Team& t, 
 enum Outcome { OUT_FOUND = 0, OUT_NONE = 1, OUT_ZERO = 2 };
 
 template <class CT, int TK>
-__device__ __noinline__ void bf_call(const BfParams& P, const Team& t, char* smem) {
-    bf_body<CT, TK, false, true>(P, t, smem);
+__device__ __noinline__ void bf_call(const BfParams& P, const Team& t) {
+    bf_body<CT, TK, false>(P, t, reinterpret_cast<char*>(smemRaw));
+}
+template <class CT, int TK>
+__device__ __noinline__ void bf_local_call(const BfParams& P, const Team& t) {
+    bf_body<CT, TK, false, 2>(P, t, nullptr);
 }
 
 // One Bellman-Ford call of the team: the lead publishes the call's state,
 // the Bellman-Ford CTAs run it, and every CTA reads its verdict after the
 // closing barrier.  False when a team barrier ran out.
 template <class CT, int TK>
-__device__ bool team_bf_call(PairJob& J, const BfParams& P, const SolveTeam& S, char* smem, bool resetError) {
+__device__ bool team_bf_call(PairJob& J, const BfParams& P, const SolveTeam& S, bool resetError) {
     if (S.lead()) {
         P.ctl->status = BF_RUNNING;
         if (resetError) P.ctl->error = 0;
     }
     if (!team_sync(S.all)) return false;
-    if (S.in_bf()) bf_call<CT, TK>(P, S.bf, smem);
+    if (S.in_bf()) {
+        if (P.localKD) bf_local_call<CT, TK>(P, S.bf);
+        else bf_call<CT, TK>(P, S.bf);
+    }
     if (!team_sync(S.all)) return false;
     if (S.lead()) {
         J.bfCalls++;
@@ -1597,7 +1698,7 @@ __device__ bool team_bf_call(PairJob& J, const BfParams& P, const SolveTeam& S, 
 // one thread of every CTA, in the same order, so every CTA takes the same
 // branches; only the lead writes the job's outputs.
 template <class CT, int TK>
-__device__ void pair_solve(PairJob& J, BfParams& P, const SolveTeam& S, char* smem) {
+__device__ void pair_solve(PairJob& J, BfParams& P, const SolveTeam& S) {
     __shared__ int sState[4];        // [1] the bound search gave up, [3] edges of the last record
     __shared__ double sRatio;
     const Team& t = S.all;
@@ -1620,7 +1721,7 @@ __device__ void pair_solve(PairJob& J, BfParams& P, const SolveTeam& S, char* sm
         const CT* c1 = reinterpret_cast<const CT*>(P.cost) + P.layerStride;
         for (long long vv = t.thread(); vv < n; vv += t.nthreads()) {
             const int v = (int)vv;
-            const int s = v >> 5, lane = v & 31;
+            const int slot = __ldg(P.nodeSlot + v), s = slot >> 5, lane = slot & 31;
             float mean = 0;
             int num = 0;
             for (int j = __ldg(P.spInter + s); j < __ldg(P.spInter + s + 1); ++j) {
@@ -1663,7 +1764,7 @@ __device__ void pair_solve(PairJob& J, BfParams& P, const SolveTeam& S, char* sm
         P.lambda = 10;
         P.ub = ubInf;
     }
-    if (!team_bf_call<CT, TK>(J, P, S, smem, true)) PGC_TEAM_FAIL();
+    if (!team_bf_call<CT, TK>(J, P, S, true)) PGC_TEAM_FAIL();
     if (*(volatile int*)&ctl->error) PGC_TEAM_FAIL();
     {
         const int st = *(volatile int*)&ctl->status;
@@ -1730,7 +1831,7 @@ __device__ void pair_solve(PairJob& J, BfParams& P, const SolveTeam& S, char* sm
             P.lambda = currentRatio;
             P.ub = ubInf;
         }
-        if (!team_bf_call<CT, TK>(J, P, S, smem, false)) PGC_TEAM_FAIL();
+        if (!team_bf_call<CT, TK>(J, P, S, false)) PGC_TEAM_FAIL();
         if (lead) J.lawlerIters++;
         if (*(volatile int*)&ctl->error) PGC_TEAM_FAIL();
         const int st = *(volatile int*)&ctl->status;
@@ -1824,10 +1925,8 @@ __device__ void pair_solve(PairJob& J, BfParams& P, const SolveTeam& S, char* sm
 // With more than one CTA per team the launch is cooperative, so that every
 // CTA of a team is resident.
 template <class CT, int TK>
-__global__ void __launch_bounds__(kBatchThreads, kBatchBlocksPerSm)
+__global__ void __launch_bounds__(kBatchThreads + 32, kBatchBlocksPerSm)
     bf_batch_kernel(PairJob* jobs, int count, int* next, unsigned* teamWords, int teamCtas, unsigned spin) {
-    extern __shared__ double4 smemRaw[];
-    char* smem = reinterpret_cast<char*>(smemRaw);
     __shared__ BfParams P;
     __shared__ int sJob, sCtas;
     const int cta = (int)(blockIdx.x % (unsigned)teamCtas);
@@ -1848,7 +1947,7 @@ __global__ void __launch_bounds__(kBatchThreads, kBatchBlocksPerSm)
         __syncthreads();
         const SolveTeam S{all, Team{cta, sCtas, &P.ctl->barCount, &P.ctl->barGen, &P.ctl->error, P.spinLimit}};
         const long long c0 = clock64();
-        pair_solve<CT, TK>(jobs[j], P, S, smem);
+        pair_solve<CT, TK>(jobs[j], P, S);
         if (lead) {
             jobs[j].candidates = P.ctl->candidates;
             jobs[j].fallbackWalks = P.ctl->fallbackWalks;
@@ -1860,7 +1959,16 @@ __global__ void __launch_bounds__(kBatchThreads, kBatchBlocksPerSm)
 }
 
 // Host-side launch helpers -------------------------------------------------
-static const void* bf_fn(int costIsF32, int timeKind, bool sharedTables) {
+static const void* bf_fn(int costIsF32, int timeKind, bool sharedTables, bool local) {
+    if (local) {
+        if (costIsF32)
+            return timeKind == 0 ? (const void*)bf_local_kernel<float, 0>
+                                 : timeKind == 1 ? (const void*)bf_local_kernel<float, 1>
+                                                 : (const void*)bf_local_kernel<float, 2>;
+        return timeKind == 0 ? (const void*)bf_local_kernel<double, 0>
+                             : timeKind == 1 ? (const void*)bf_local_kernel<double, 1>
+                                             : (const void*)bf_local_kernel<double, 2>;
+    }
     if (sharedTables) {
         if (costIsF32)
             return timeKind == 0 ? (const void*)bf_kernel<float, 0, true>
@@ -1938,7 +2046,7 @@ static cudaError_t max_blocks_per_sm(const void* fn, int threads, size_t smemByt
 cudaError_t launch_bf(const BfParams& p, int costIsF32, int timeKind, int blocks, int threads, bool cooperative,
                       bool sharedTables, size_t smemBytes, cudaStream_t stream) {
     void* args[] = {(void*)&p};
-    const void* fn = bf_fn(costIsF32, timeKind, sharedTables);
+    const void* fn = bf_fn(costIsF32, timeKind, sharedTables, p.localKD > 0);
     const cudaError_t e = allow_max_dynamic_smem(fn);
     if (e != cudaSuccess) return e;
     note_launch();
@@ -1946,11 +2054,22 @@ cudaError_t launch_bf(const BfParams& p, int costIsF32, int timeKind, int blocks
     return cudaLaunchKernel(fn, dim3(blocks), dim3(threads), args, smemBytes, stream);
 }
 
-cudaError_t bf_max_coop_blocks(int costIsF32, int timeKind, int threads, size_t smemBytes, int* blocksPerSm) {
-    const void* fn = bf_fn(costIsF32, timeKind, false);
+cudaError_t bf_max_coop_blocks(int costIsF32, int timeKind, bool local, int threads, size_t smemBytes,
+                               int* blocksPerSm) {
+    const void* fn = bf_fn(costIsF32, timeKind, false, local);
     const cudaError_t e = allow_max_dynamic_smem(fn);
     if (e != cudaSuccess) return e;
     return max_blocks_per_sm(fn, threads, smemBytes, blocksPerSm);
+}
+
+cudaError_t launch_local_plan(const LocalPlanArgs& a, int maxCtaSlices, cudaStream_t stream) {
+    const cudaError_t e = allow_max_dynamic_smem((const void*)local_plan_kernel);
+    if (e != cudaSuccess) return e;
+    note_launch();
+    local_used_kernel<<<148, 512, 0, stream>>>(a);
+    note_launch();
+    local_plan_kernel<<<a.ncta, 512, (size_t)(2 * a.nslices + maxCtaSlices) * 4, stream>>>(a);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_extract_path(const BfParams& p, int v, cudaStream_t stream) {

@@ -1025,11 +1025,11 @@ __global__ void export_kernel(const double* col, double* out, int cols, int c, l
 // CT: the fp64 column or its exact fp32 copy (the same values).
 template <class CT>
 __global__ void layer1_mean_kernel(const CT* cost, long long layerStride, long long interEntries, int n,
-                                   int nslices, const int* spInter, const int* spIntra, const int* srcInter,
+                                   const int* nodeSlot, const int* spInter, const int* spIntra, const int* srcInter,
                                    const int* srcIntra, float* meanOut, int* countOut) {
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= n) return;
-    const int s = v >> 5, lane = v & 31;
+    const int slot = nodeSlot[v], s = slot >> 5, lane = slot & 31;
     const CT* c1 = cost + layerStride;  // layer 1
     float mean = 0;
     int num = 0;
@@ -1047,7 +1047,6 @@ __global__ void layer1_mean_kernel(const CT* cost, long long layerStride, long l
     }
     meanOut[v] = mean / (float)num;
     countOut[v] = num;
-    (void)nslices;
 }
 
 // ---------------------------------------------------------------------------
@@ -1525,19 +1524,19 @@ cudaError_t launch_import(const double* in, double* col, int cols, int c, long l
                                                        ti, tr);
     return cudaGetLastError();
 }
-cudaError_t launch_layer1_mean(const double* cost, long long layerStride, long long interEntries, int n, int nslices,
-                               const int* spI, const int* spA, const int* srcI, const int* srcA, float* meanOut,
-                               int* countOut, cudaStream_t s) {
+cudaError_t launch_layer1_mean(const double* cost, long long layerStride, long long interEntries, int n,
+                               const int* nodeSlot, const int* spI, const int* spA, const int* srcI, const int* srcA,
+                               float* meanOut, int* countOut, cudaStream_t s) {
     note_launch();
-    layer1_mean_kernel<double><<<(n + 255) / 256, 256, 0, s>>>(cost, layerStride, interEntries, n, nslices, spI, spA,
+    layer1_mean_kernel<double><<<(n + 255) / 256, 256, 0, s>>>(cost, layerStride, interEntries, n, nodeSlot, spI, spA,
                                                                srcI, srcA, meanOut, countOut);
     return cudaGetLastError();
 }
-cudaError_t launch_layer1_mean(const float* cost, long long layerStride, long long interEntries, int n, int nslices,
-                               const int* spI, const int* spA, const int* srcI, const int* srcA, float* meanOut,
-                               int* countOut, cudaStream_t s) {
+cudaError_t launch_layer1_mean(const float* cost, long long layerStride, long long interEntries, int n,
+                               const int* nodeSlot, const int* spI, const int* spA, const int* srcI, const int* srcA,
+                               float* meanOut, int* countOut, cudaStream_t s) {
     note_launch();
-    layer1_mean_kernel<float><<<(n + 255) / 256, 256, 0, s>>>(cost, layerStride, interEntries, n, nslices, spI, spA,
+    layer1_mean_kernel<float><<<(n + 255) / 256, 256, 0, s>>>(cost, layerStride, interEntries, n, nodeSlot, spI, spA,
                                                               srcI, srcA, meanOut, countOut);
     return cudaGetLastError();
 }

@@ -314,7 +314,7 @@ class Graph {
     bool generated = false;
     LayerTemplate T;
     int ncols = 1;
-    DBuf<int> dSp[2], dSrc[2], dTedge[2], dSrcDummy, dEX, dEY, dESrc, dETrgt, dEXcols;
+    DBuf<int> dSlotNode, dNodeSlot, dSp[2], dSrc[2], dTedge[2], dSrcDummy, dEX, dEY, dESrc, dETrgt, dEXcols;
     DBuf<int8_t> dEYpat, dENext;
     DBuf<double> dVX, dVY, dFD, dNX, dNY;
     DBuf<double4> dQuat;
@@ -467,15 +467,31 @@ class Graph {
         const void* time;
         double tconst;
         int blocks, threads;
+        int extraThreads;   // launched on top: the staging warp of teams on local tables
         bool coop;
         bool sharedTables;  // single CTA keeping its DP records in shared memory
         int flagSync;       // neighbour hand-offs between steps (multi-CTA teams)
         int maxCtaSlices;   // most slices any CTA owns
         int rowCap;         // rows a step buffer holds (0: streams read in place)
         int stageSrcOnly;   // the buffers hold source indices only
+        int localKD;        // depths of the per-CTA local tables (0: records in global memory)
+        int hopBits;
         size_t smemBytes;   // dynamic shared memory per CTA
     };
     Run prepare_run(int K, bool ratio);
+    bool plan_local(Run& r, int blocks, size_t smemCap);
+    // the local tables' plan of the partition in ctaCut (local_plan_kernel)
+    struct LocalPlan {
+        std::vector<int> cut;
+        int parts = 0, cap = 0;
+        int L = 0, halo = 0, rows[2] = {0, 0}, maxSlices = 0;
+        bool fits = false;  // no CTA's halo or table outgrew the plan
+    } localPlan;
+    DBuf<unsigned short> wLsrc[2];
+    DBuf<unsigned> wHaloSlot, wExposed;
+    DBuf<int> wLocalCounts;
+    DBuf<unsigned char> wSliceUsed;
+    DBuf<uint4> wXbuf;
     // batch mode of prepare_run: a team of up to batchCtas CTAs of
     // batchThreads threads, DP records in global memory, staging only within
     // batchSmemCap bytes
@@ -508,7 +524,7 @@ class Graph {
 // The product-graph topology depends only on EX, EY and the two graph flags,
 // all fixed at construction; it is built and uploaded once.
 void Graph::upload_template() {
-    const std::string err = build_template(EX.data(), nex, EY.data(), ney, nvx, conj, prune, T);
+    const std::string err = build_template(EX.data(), nex, EY.data(), ney, nvx, conj, prune, T, true);
     if (!err.empty()) throw Failure(PGC_ERR_ARG, err);
     for (int64_t i = 0; i < 2 * ney; ++i)
         if (EY[(size_t)i] >= nvy) throw Failure(PGC_ERR_ARG, "EY refers to a vertex outside VY");
@@ -518,6 +534,8 @@ void Graph::upload_template() {
         dSrc[p].upload(T.src[p].data(), T.src[p].size(), s);
         dTedge[p].upload(T.tedge[p].data(), T.tedge[p].size(), s);
     }
+    dSlotNode.upload(T.slotNode.data(), T.slotNode.size(), s);
+    dNodeSlot.upload(T.nodeSlot.data(), T.nodeSlot.size(), s);
     // The closing layer's source list differs from the interlayer one only
     // with two layers; otherwise the kernels read the interlayer list.
     if (T.nY == 2) dSrcDummy.upload(T.srcDummy.data(), T.srcDummy.size(), s);
@@ -829,6 +847,10 @@ Graph::Run Graph::prepare_run(int K, bool ratio) {
         r.threads = batchThreads;
         r.blocks = std::max(1, std::min(batchCtas, T.nslices));
         r.coop = false;
+        if (plan_local(r, r.blocks, batchSmemCap)) {
+            ensure_workspace(K, std::max(r.blocks, batchCtas));
+            return r;
+        }
         r.sharedTables = false;
         r.flagSync = r.blocks > 1 && env_int("PGC_BF_FLAGS", 1) ? 1 : 0;
         int maxSl = 0, rowCap = 0;
@@ -858,6 +880,34 @@ Graph::Run Graph::prepare_run(int K, bool ratio) {
     if (!envThreads) envThreads = shapeThreads;
     if (envThreads && (envThreads < 32 || envThreads > kBfThreads || envThreads % 32 != 0))
         throw Failure(PGC_ERR_ARG, "PGC_BF_THREADS must be a multiple of 32 in [32, 640]");
+    {
+        // Teams on local tables: one CTA while a step's relaxation is shorter
+        // than an exchange, else CTAs of a few slices each, up to one per SM.
+        int active = 0;
+        for (int s = 0; s < T.nslices; ++s)
+            if (T.sp[INTER][(size_t)s + 1] > T.sp[INTER][(size_t)s]) ++active;
+        int lb = envBlocks;
+        if (lb <= 0) {
+            lb = active <= env_int("PGC_BF_LOCAL_ONE", 24) ? 1 : (active + env_int("PGC_BF_LOCAL_SL", 4) - 1) / env_int("PGC_BF_LOCAL_SL", 4);
+            if (teamCap > 0) lb = std::min(lb, teamCap);
+        }
+        lb = std::max(1, std::min({lb, T.nslices, sms}));
+        // relaxing warps: one per slice of the largest share, at most 20; the
+        // launch adds one that stages the streams
+        r.threads = envThreads ? envThreads
+                               : std::min(kBfThreads, 32 * std::max(2, (active + lb - 1) / lb));
+        if (plan_local(r, lb, smemCap)) {
+            r.extraThreads = 32;
+            if (r.blocks > 1) {
+                int perSm = 0;
+                PGC_CUDA(bf_max_coop_blocks(r.costF32, r.timeKind, true, r.threads + 32, r.smemBytes, &perSm));
+                if (perSm < 1) throw Failure(PGC_ERR_CUDA, "the Bellman-Ford kernel cannot be resident with its shared memory");
+            }
+            r.coop = r.blocks > 1;
+            ensure_workspace(K, r.blocks);
+            return r;
+        }
+    }
     int maxSl = 0, rowCap = 0;
     int blocks = envBlocks;
     if (blocks <= 0 && T.nslices <= env_int("PGC_BF_SINGLE_CTA_SLICES", 64) &&
@@ -873,7 +923,7 @@ Graph::Run Graph::prepare_run(int K, bool ratio) {
                      tables + bf_stage_offset(T.nslices) <= smemCap;
     if (blocks > 1) {
         int perSm = 0;
-        PGC_CUDA(bf_max_coop_blocks(r.costF32, r.timeKind, r.threads, 0, &perSm));
+        PGC_CUDA(bf_max_coop_blocks(r.costF32, r.timeKind, false, r.threads, 0, &perSm));
         if (perSm < 1) throw Failure(PGC_ERR_CUDA, "the Bellman-Ford kernel cannot be resident with this block size");
         blocks = std::min(blocks, sms * perSm);
     }
@@ -900,7 +950,7 @@ Graph::Run Graph::prepare_run(int K, bool ratio) {
     if (r.smemBytes > smemCap) throw Failure(PGC_ERR_ARG, "the product graph's DP tables do not fit shared memory");
     if (blocks > 1) {
         int perSm = 0;
-        PGC_CUDA(bf_max_coop_blocks(r.costF32, r.timeKind, r.threads, r.smemBytes, &perSm));
+        PGC_CUDA(bf_max_coop_blocks(r.costF32, r.timeKind, false, r.threads, r.smemBytes, &perSm));
         if (perSm < 1) throw Failure(PGC_ERR_CUDA, "the Bellman-Ford kernel cannot be resident with its shared memory");
         if (blocks > sms * perSm) {
             // fewer CTAs fit with this much shared memory: read in place
@@ -919,6 +969,102 @@ Graph::Run Graph::prepare_run(int K, bool ratio) {
     if (cut.size() != (size_t)blocks + 1) stage_need(blocks, maxSl, rowCap);
     upload_cta_slices(cut, K, r.threads / 32);
     return r;
+}
+
+// A team of `blocks` CTAs that sweeps on per-CTA local tables
+// (bf_local.cuh), when the graph allows it: at most four source depths, three
+// layers or more, slots that the plan's bitmaps hold, path origins and
+// lengths that share 32 bits, and tables that fit `smemCap`.  Fills the run's
+// team and shared-memory fields; false: the sweeps work in global memory.
+bool Graph::plan_local(Run& r, int blocks, size_t smemCap) {
+    r.localKD = 0;
+    const int KD = T.entries[INTRA] == 0 ? 1 : r.K, nslots = T.nslices * 32;
+    if (KD > 4 || T.nY < 3 || nslots > kLocalMaxSlots) return false;
+    if (!env_int("PGC_BF_LOCAL", 1) || !env_int("PGC_BF_FLAGS", 1) || !env_int("PGC_BF_STAGE", 1) ||
+        env_int("PGC_BF_STAGE_SRC", 1) != 1)
+        return false;
+    int hopBits = 1;
+    while (((long long)1 << hopBits) < (long long)(T.nY + 1) * KD + 2) ++hopBits;
+    if (hopBits > 24 || (long long)T.n + 2 > (1LL << (32 - hopBits))) return false;
+    const int parts = KD > 1 ? 2 : 1;
+    const std::vector<int> cut = plan_even_cuts(T, blocks, r.K);
+    LocalPlan& q = localPlan;
+    if (q.parts != parts || q.cut != cut) {
+        q.cut.clear();
+        q.maxSlices = 0;
+        q.rows[0] = q.rows[1] = 0;
+        for (int c = 0; c < blocks; ++c) {
+            const int a = cut[(size_t)c], b = cut[(size_t)c + 1];
+            q.maxSlices = std::max(q.maxSlices, b - a);
+            for (int p = 0; p < parts; ++p) q.rows[p] = std::max(q.rows[p], T.sp[p][(size_t)b] - T.sp[p][(size_t)a]);
+        }
+        DeviceInfo info{};
+        PGC_CUDA(device_info(device, &info));
+        const size_t smemOpt = (size_t)std::max(0, info.smemOptin);
+        if ((size_t)(2 * T.nslices + q.maxSlices) * 4 + 8192 > smemOpt) return false;
+        q.cap = blocks > 1 ? std::min(nslots, 16384) : 1;
+        for (int p = 0; p < 2; ++p) wLsrc[p].alloc((size_t)T.entries[p] + 2);
+        wHaloSlot.alloc((size_t)blocks * q.cap);
+        wExposed.alloc((size_t)T.nslices);
+        wSliceUsed.alloc((size_t)T.nslices);
+        wLocalCounts.alloc((size_t)2 * blocks);
+        PGC_CUDA(cudaMemsetAsync(wExposed.p, 0, (size_t)T.nslices * 4, stream));
+        PGC_CUDA(cudaMemsetAsync(wSliceUsed.p, 0, (size_t)T.nslices, stream));
+        upload_cta_slices(cut, r.K, -1);
+        LocalPlanArgs a{};
+        a.nslices = T.nslices;
+        a.ncta = blocks;
+        a.parts = parts;
+        a.ctaSlice = wCtaSlice.p;
+        for (int p = 0; p < 2; ++p) {
+            a.sp[p] = dSp[p].p;
+            a.src[p] = dSrc[p].p;
+            a.entries[p] = T.entries[p];
+            a.lsrc[p] = wLsrc[p].p;
+        }
+        a.nodeSlot = dNodeSlot.p;
+        a.used = wSliceUsed.p;
+        a.haloSlot = wHaloSlot.p;
+        a.haloCap = q.cap;
+        a.counts = wLocalCounts.p;
+        a.exposed = wExposed.p;
+        PGC_CUDA(launch_local_plan(a, q.maxSlices, stream));
+        stats.launches += 2;
+        std::vector<int> counts((size_t)2 * blocks);
+        d2h(counts.data(), wLocalCounts.p, sizeof(int) * counts.size());
+        PGC_CUDA(sync_stream());
+        q.L = q.halo = 0;
+        q.fits = true;
+        for (int c = 0; c < blocks; ++c) {
+            const int halo = counts[(size_t)c], L = 32 * counts[(size_t)(blocks + c)] + halo + 1;
+            q.halo = std::max(q.halo, halo);
+            q.L = std::max(q.L, L);
+            if (halo > q.cap || L > 0xffff) q.fits = false;
+        }
+        q.parts = parts;
+        q.cut = cut;
+    } else {
+        upload_cta_slices(cut, r.K, -1);
+    }
+    if (!q.fits) return false;
+    const int costBytes = r.costF32 ? 4 : 8, timeBytes = r.timeKind == 1 ? 4 : r.timeKind == 2 ? 8 : 0;
+    const size_t tables = local_layout(q.maxSlices, q.L, q.halo, q.rows[0], q.rows[1], KD).total;
+    r.rowCap = std::max(1, std::max(q.rows[0], q.rows[1]));
+    r.smemBytes = tables + (size_t)2 * r.rowCap * 32 * (costBytes + timeBytes);
+    if (r.smemBytes > smemCap) {
+        r.rowCap = 0;  // the streams are read in place, prefetched into L2
+        r.smemBytes = tables;
+        if (tables > smemCap) return false;
+    }
+    if (blocks > 1) wXbuf.alloc((size_t)2 * KD * nslots);
+    r.localKD = KD;
+    r.hopBits = hopBits;
+    r.blocks = blocks;
+    r.sharedTables = false;
+    r.flagSync = 1;
+    r.maxCtaSlices = q.maxSlices;
+    r.stageSrcOnly = 0;
+    return true;
 }
 
 // CTA slice ranges of the team (plan_cta_cuts), cached per (blocks, K,
@@ -1007,6 +1153,25 @@ BfParams Graph::params(const Run& r, int mode, int branchId, double lambda, doub
     p.K = r.K;
     p.Kp = r.Kp;
     p.nslices = T.nslices;
+    p.nslots = T.nslices * 32;
+    p.slotNode = dSlotNode.p;
+    p.nodeSlot = dNodeSlot.p;
+    p.localKD = r.localKD;
+    if (r.localKD) {
+        p.localL = localPlan.L;
+        p.localHalo = localPlan.halo;
+        p.localRows[INTER] = localPlan.rows[INTER];
+        p.localRows[INTRA] = localPlan.rows[INTRA];
+        p.hopBits = r.hopBits;
+        p.lsrc[INTER] = wLsrc[INTER].p;
+        p.lsrc[INTRA] = wLsrc[INTRA].p;
+        p.haloSlot = wHaloSlot.p;
+        p.haloCnt = wLocalCounts.p;
+        p.haloCap = localPlan.cap;
+        p.exposed = wExposed.p;
+        p.sliceUsed = wSliceUsed.p;
+        p.xbuf = wXbuf.p;
+    }
     p.numNodes = numNodes();
     p.spInter = dSp[INTER].p;
     p.spIntra = dSp[INTRA].p;
@@ -1074,7 +1239,7 @@ Control Graph::launch_bf_call(const Run& r, const BfParams& p) {
     }
     cudaEvent_t e0 = timeEvents[0], e1 = timeEvents[1];
     PGC_CUDA(cudaEventRecord(e0, stream));
-    PGC_CUDA(launch_bf(p, r.costF32, r.timeKind, r.blocks, r.threads, r.coop, r.sharedTables, r.smemBytes, stream));
+    PGC_CUDA(launch_bf(p, r.costF32, r.timeKind, r.blocks, r.threads + r.extraThreads, r.coop, r.sharedTables, r.smemBytes, stream));
     PGC_CUDA(cudaEventRecord(e1, stream));
     stats.launches++;
     d2h(&c, wCtl.p, sizeof(Control));
@@ -1140,6 +1305,7 @@ void Graph::lookup_pairs(const std::vector<int>& src, const std::vector<int>& tr
     LookupArgs a{};
     a.n = T.n;
     a.nY = T.nY;
+    a.nodeSlot = dNodeSlot.p;
     a.numNodes = numNodes();
     a.eBlock = T.eBlock;
     a.spInter = dSp[INTER].p;
@@ -1253,10 +1419,10 @@ void Graph::solve_ratio_rescaled(int K) {
         std::vector<float> mean((size_t)n);
         std::vector<int> cnt((size_t)n);
         if (e64Stale[0])
-            PGC_CUDA(launch_layer1_mean(e32[0].p, T.layerStride(), T.entries[INTER], n, T.nslices, dSp[INTER].p,
+            PGC_CUDA(launch_layer1_mean(e32[0].p, T.layerStride(), T.entries[INTER], n, dNodeSlot.p, dSp[INTER].p,
                                         dSp[INTRA].p, dSrc[INTER].p, dSrc[INTRA].p, wMean.p, wCandStat.p, stream));
         else
-            PGC_CUDA(launch_layer1_mean(e64[0].p, T.layerStride(), T.entries[INTER], n, T.nslices, dSp[INTER].p,
+            PGC_CUDA(launch_layer1_mean(e64[0].p, T.layerStride(), T.entries[INTER], n, dNodeSlot.p, dSp[INTER].p,
                                         dSp[INTRA].p, dSrc[INTER].p, dSrc[INTRA].p, wMean.p, wCandStat.p, stream));
         stats.launches++;
         d2h(mean.data(), wMean.p, sizeof(float) * n);
@@ -1479,6 +1645,7 @@ void Graph::batch_begin(int K, PairJob& J, int threads, int ctas, size_t smemCap
     LookupArgs& a = J.lk;
     a.n = T.n;
     a.nY = T.nY;
+    a.nodeSlot = dNodeSlot.p;
     a.numNodes = numNodes();
     a.eBlock = T.eBlock;
     a.spInter = dSp[INTER].p;
@@ -2383,12 +2550,26 @@ int pgc_solve_batch(pgc_graph* const* graphs, int64_t count, const char* solver,
             // device.  The costs are generated and rescaled per graph by the
             // workers first; graphs whose first branch's cycle wraps are
             // finished on the host afterwards, with branch and bound.
-            const int threads = pgc::kBatchThreads;
-            const size_t smemCap = (size_t)std::max(0, info.smemOptin / pgc::kBatchBlocksPerSm - 2048);
-            // CTAs per team (PGC_BATCH_TEAM, default 8): a team relaxes a
-            // graph's steps side by side, so more CTAs per graph shorten each
-            // solve; fewer overlap more graphs' latencies
-            int team = ctas_per_graph > 0 ? ctas_per_graph : pgc::env_int("PGC_BATCH_TEAM", 8);
+            const size_t smemCap = (size_t)std::max(0, info.smemOptin / pgc::kBatchBlocksPerSm - 2560);
+            // Relaxing threads per CTA: 20 warps, or 8 for graphs whose mean
+            // fits 8 slices.  CTAs per team (ctas_per_graph, else
+            // PGC_BATCH_TEAM, else a mean share of one slice per warp, as a
+            // power of two of at most 16): a team relaxes a graph's steps side
+            // by side, so more CTAs per graph shorten each solve; fewer solve
+            // more graphs at once.
+            double slices = 0;
+            int64_t live = 0;
+            for (int64_t i = 0; i < count; ++i) {
+                if (!graphs[i]) continue;
+                const Graph& g = graphs[i]->g;
+                slices += g.conj ? 3.0 * (double)g.nex / 32 : (double)g.nvx / 32;
+                ++live;
+            }
+            slices /= (double)std::max<int64_t>(1, live);
+            const int threads = slices <= 8 ? 256 : pgc::kBatchThreads;
+            int team = ctas_per_graph > 0 ? ctas_per_graph : pgc::env_int("PGC_BATCH_TEAM", 0);
+            if (team <= 0)
+                for (team = 1; team < 16 && team * (threads / 32) < slices;) team *= 2;
             team = std::max(1, std::min(team, sms * pgc::kBatchBlocksPerSm));
             const unsigned spin = (unsigned)std::max(1, pgc::env_int("PGC_BF_SPIN_LIMIT", (int)pgc::kDefaultSpinLimit));
             std::vector<PairJob> jobs((size_t)count);
@@ -2462,7 +2643,7 @@ int pgc_solve_batch(pgc_graph* const* graphs, int64_t count, const char* solver,
                     while (k1 < order.size() && costF32[(size_t)order[k1]] == cf && timeKind[(size_t)order[k1]] == tk)
                         smem = std::max(smem, smemNeed[(size_t)order[k1++]]);
                     int perSm = 0;
-                    PGC_CUDA(pgc::bf_batch_max_blocks(cf, tk, threads, smem, &perSm));
+                    PGC_CUDA(pgc::bf_batch_max_blocks(cf, tk, threads + 32, smem, &perSm));
                     if (perSm < 1) throw Failure(PGC_ERR_CUDA, "the batched solve kernel cannot be resident");
                     // whole teams, all resident (the launch is cooperative
                     // when a team has more than one CTA)
@@ -2474,7 +2655,7 @@ int pgc_solve_batch(pgc_graph* const* graphs, int64_t count, const char* solver,
                     g_batchProfile[6] = threads;
                     g_batchProfile[7] = std::max(g_batchProfile[7], (double)smem);
                     PGC_CUDA(pgc::launch_bf_batch(dJobs.p + k0, (int)(k1 - k0), dNext.p + grp % 8, dTeamWords.p, g,
-                                                  spin, cf, tk, blocks, threads, smem, bs));
+                                                  spin, cf, tk, blocks, threads + 32, smem, bs));
                     k0 = k1;
                 }
                 PGC_CUDA(cudaMemcpyAsync(packed.data(), dJobs.p, sizeof(PairJob) * packed.size(),
