@@ -505,7 +505,7 @@ __device__ double4 frame_quaternion(const double v2[3], const double n2[3], cons
 // i, or i - 1 for the degenerate-2d nodes |EX| <= j < 2|EX| of an unpruned
 // graph.  The reference stores 3|EX| frames per layer; every one of them is
 // a copy of frame (Y edge, X edge) of the |EX| x nY distinct ones, which is
-// all that is computed here (quat_index maps a node to its frame).
+// all that is computed here.
 __global__ void quaternion_kernel(QuatArgs a) {
     const long long total = (long long)a.nY * a.nEX;
     for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
@@ -543,135 +543,161 @@ __device__ __forceinline__ double4 ldg_quat(const double4* q) {
     return make_double4(lo.x, lo.y, hi.x, hi.y);
 }
 
-// Frame of conjugate node j of layer i (see quaternion_kernel).
-__device__ __forceinline__ long long quat_index(const EnergyArgs& a, int i, int j) {
-    const int e3 = j % a.quatEX;
-    const int i2 = (j >= a.quatEX && j < 2 * a.quatEX && !a.quatPrune) ? (i + a.nY - 1) % a.nY : i;
-    return (long long)i2 * a.quatEX + e3;
-}
-
-// Work item: one block of template positions x a chunk of layers.  A thread
-// keeps its position -- template edge, Y pattern, X columns, frame indices,
-// the X half of the line integral -- and walks the chunk's layers, so per
-// layer it reads only the layer's Y edge and the fd entry; the stores of a
-// warp stay 32 consecutive entries of one layer.  Every value is computed
-// with the same operations in the same order as per entry.
+// Work item: a block of template positions x a chunk of layers.  A thread
+// keeps two positions, the same lane of two consecutive rows -- template edge,
+// Y pattern, X columns, frames, the X half of the line integral -- and walks
+// the chunk's layers, so per layer it reads only the layer's Y edge, the fd
+// entry and the frames; the stores of a warp stay 32 consecutive entries of
+// one layer.  In-edges come in pairs that leave the same X edge (a node and
+// its degenerate copy), so the two rows often join the same two frames: their
+// distance and its robust loss, an arc cosine and two powers, are then
+// computed once (and the fd entry, of the same target, read once).  Every
+// value is computed with the same operations in the same order as per entry.
 constexpr int kHoLayerChunk = 16;
 
-__global__ void ho_energy_kernel(EnergyArgs a) {
+struct HoPosition {
+    bool on, isInter;
+    int pat, x1, x2;
+    int src, srcBack, trgt, trgtNext, trgtBack;  // frames: X edge, and layers behind or ahead of the block's
+    double dxx[3];
+};
+
+__global__ void __launch_bounds__(256) ho_energy_kernel(EnergyArgs a) {
     extern __shared__ unsigned int topSh[];  // [2][kTopBins] when a.hist0
     DigitRun r0, r1;
     top_digit_begin(a, topSh);
     const double nan = __longlong_as_double(0x7ff8000000000000LL);
     const double twoPi = 2 * 3.14159265358979323846;
     const bool needLi = (a.costMode == LENGTH || a.timeMode == LENGTH);
+    const int cm = a.costMode, tm = a.timeMode;
     // Without quaternions every SO(3) distance is 0: its robust loss is the
     // same number for every edge, computed once per thread by the same code.
     const double rl0 = robust_loss(a, 0.0);
     const int stride = (int)a.layerStride, inter = (int)a.interEntries, layers = a.nY + 1;
-    const int posBlocks = (stride + (int)blockDim.x - 1) / (int)blockDim.x;
+    const int perBlock = 2 * (int)blockDim.x;
+    const int posBlocks = (stride + perBlock - 1) / perBlock;
     const int chunks = (layers + kHoLayerChunk - 1) / kHoLayerChunk;
     const long long items = (long long)posBlocks * chunks;
     for (long long it = blockIdx.x; it < items; it += gridDim.x) {
         const int lc = (int)(it / posBlocks);
-        const int pos = (int)(it - (long long)lc * posBlocks) * (int)blockDim.x + (int)threadIdx.x;
-        if (pos >= stride) continue;
+        const int pos0 = (int)(it - (long long)lc * posBlocks) * perBlock + (int)(threadIdx.x >> 5) * 64 +
+                         (int)(threadIdx.x & 31);
+        if (pos0 >= stride) continue;
         const int l0 = lc * kHoLayerChunk, l1 = min(l0 + kHoLayerChunk, layers);
-        const bool isInter = pos < inter;
-        const int t = isInter ? __ldg(a.tedgeInter + pos) : __ldg(a.tedgeIntra + (pos - inter));
-        if (t < 0) {
-            for (int l = l0; l < l1; ++l) {
-                const long long idx = (long long)l * stride + pos;
-                a.out0[idx] = nan;
-                if (a.out1) a.out1[idx] = nan;
-            }
-            continue;
-        }
-        const int pat = __ldg(a.eY + t);
-        const int x0 = __ldg(a.eX + 3 * t), x1 = __ldg(a.eX + 3 * t + 1), x2 = __ldg(a.eX + 3 * t + 2);
-        double dxx[3] = {0.0, 0.0, 0.0};
-        if (needLi) {
+        HoPosition P[2];
 #pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                const double dx = __ldg(a.VX + 3 * x0 + j) - __ldg(a.VX + 3 * x1 + j);
-                dxx[j] = dx * dx;
-            }
-        }
-        int eSrc = 0, eTrgt = 0, eNext = 0;
-        if (a.quat) {
-            eSrc = __ldg(a.eSrc + t);
-            eTrgt = __ldg(a.eTrgt + t);
-            eNext = __ldg(a.eNext + t);
-        }
-        const double* fdRow = a.FD + (long long)x2 * a.nvy;
-        for (int l = l0; l < l1; ++l) {
-            const long long idx = (long long)l * stride + pos;
-            if (isInter ? l < 1 : l >= a.nY) {  // no edge in this layer's slot
-                a.out0[idx] = nan;
-                if (a.out1) a.out1[idx] = nan;
-                continue;
-            }
-            const int b = isInter ? l - 1 : l;
-            const int s2 = __ldg(a.EY + 2 * b), m2 = __ldg(a.EY + 2 * b + 1);
-            const int t2 = __ldg(a.EY + 2 * ((b + 1) % a.nY) + 1);
-            int y0, y1, y2;
-            switch (pat) {
-                case 2: y0 = s2; y1 = s2; y2 = s2; break;
-                case 3: y0 = s2; y1 = s2; y2 = m2; break;
-                case 4: y0 = s2; y1 = m2; y2 = t2; break;
-                default: y0 = s2; y1 = m2; y2 = m2; break;
-            }
-            double so3 = 0.0;
-            if (a.quat) {
-                const long long q0 = quat_index(a, b, eSrc);
-                const long long q1 = quat_index(a, (b + eNext) % a.nY, eTrgt);
-                so3 = so3_distance(ldg_quat(a.quat + q0), ldg_quat(a.quat + q1));
-            }
-            const double rl = a.quat ? robust_loss(a, so3) : rl0;
-            const double fd = __ldg(fdRow + y2);
-            double li = 0.0;
-            if (needLi) {  // line_integral's sum, in its order
+        for (int u = 0; u < 2; ++u) {
+            HoPosition& q = P[u];
+            const int pos = pos0 + 32 * u;
+            q.isInter = pos < inter;
+            const int t = pos >= stride ? -1
+                                        : q.isInter ? __ldg(a.tedgeInter + pos) : __ldg(a.tedgeIntra + (pos - inter));
+            q.on = t >= 0;
+            if (!q.on) continue;
+            q.pat = __ldg(a.eY + t);
+            const int x0 = __ldg(a.eX + 3 * t);
+            q.x1 = __ldg(a.eX + 3 * t + 1);
+            q.x2 = __ldg(a.eX + 3 * t + 2);
+            if (needLi) {
 #pragma unroll
                 for (int j = 0; j < 3; ++j) {
-                    const double dy = __ldg(a.VY + 3 * y0 + j) - __ldg(a.VY + 3 * y1 + j);
-                    li = li + dy * dy;
-                    li = li + dxx[j];
+                    const double dx = __ldg(a.VX + 3 * x0 + j) - __ldg(a.VX + 3 * q.x1 + j);
+                    q.dxx[j] = dx * dx;
                 }
-                li = sqrt(li);
             }
-            const bool degenerate = (y2 == y1 || x2 == x1);
-            const int cm = a.costMode, tm = a.timeMode;
-            double c0 = 0, c1 = 0;
-            if (cm == VANILLA && tm == VANILLA) {
-                c0 = rl + fd;
-            } else if (cm == VANILLA && tm == LENGTH) {
-                c0 = rl + fd;
-                c1 = li;
-            } else if (cm == LENGTH && tm == VANILLA) {
-                c0 = li;
-            } else if (cm == VANILLA && tm == PENALISE_DEGENERATE) {
-                c0 = rl + fd;
-                c1 = degenerate ? 0.1 : 1;
-            } else if (cm == PENALISE_DEGENERATE && tm == VANILLA) {
-                c0 = degenerate ? 0.1 : 1;
-            } else if (cm == FEATURE && tm == SO3_PLAIN) {
-                c0 = fd;
-                c1 = fmax(0.0, twoPi - so3);
-            } else if (cm == FEATURE && tm == SO3_ROBUST) {
-                c0 = fd;
-                c1 = fmax(0.0, a.maxSO3 - rl);
-            } else if (cm == SO3_ROBUST && tm == FEATURE) {
-                c0 = rl;
-                c1 = fmax(0.0, a.maxFd - fd);
-            } else {  // SO3_PLAIN, FEATURE
-                c0 = so3;
-                c1 = fmax(0.0, a.maxFd - fd);
+            if (a.quat) {
+                // the node's X edge, one layer back for the
+                // degenerate-2d nodes of an unpruned graph
+                const int s = __ldg(a.eSrc + t), g = __ldg(a.eTrgt + t);
+                q.src = s % a.quatEX;
+                q.srcBack = s >= a.quatEX && s < 2 * a.quatEX && !a.quatPrune;
+                q.trgt = g % a.quatEX;
+                q.trgtBack = g >= a.quatEX && g < 2 * a.quatEX && !a.quatPrune;
+                q.trgtNext = __ldg(a.eNext + t);
             }
-            a.out0[idx] = c0;
-            if (a.out1) a.out1[idx] = c1;
-            if (a.hist0) {
-                count_top_digit(topSh, r0, c0);
-                if (a.hist1) count_top_digit(topSh + kTopBins, r1, c1);
+        }
+        const bool both = P[0].on && P[1].on && P[0].isInter == P[1].isInter;
+        const bool sameFrames = both && a.quat && P[0].src == P[1].src && P[0].srcBack == P[1].srcBack &&
+                                P[0].trgt == P[1].trgt && P[0].trgtBack == P[1].trgtBack &&
+                                P[0].trgtNext == P[1].trgtNext;
+        const bool sameFd = both && P[0].x2 == P[1].x2 && P[0].pat == P[1].pat;
+        for (int l = l0; l < l1; ++l) {
+            double so3 = 0.0, rl = rl0, fd = 0.0;
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const HoPosition& q = P[u];
+                const int pos = pos0 + 32 * u;
+                if (pos >= stride) break;
+                const long long idx = (long long)l * stride + pos;
+                if (!q.on || (q.isInter ? l < 1 : l >= a.nY)) {  // no edge in this layer's slot
+                    a.out0[idx] = nan;
+                    if (a.out1) a.out1[idx] = nan;
+                    continue;
+                }
+                const int b = q.isInter ? l - 1 : l;
+                const int s2 = __ldg(a.EY + 2 * b), m2 = __ldg(a.EY + 2 * b + 1);
+                const int t2 = __ldg(a.EY + 2 * (b + 1 == a.nY ? 0 : b + 1) + 1);
+                int y0, y1, y2;
+                switch (q.pat) {
+                    case 2: y0 = s2; y1 = s2; y2 = s2; break;
+                    case 3: y0 = s2; y1 = s2; y2 = m2; break;
+                    case 4: y0 = s2; y1 = m2; y2 = t2; break;
+                    default: y0 = s2; y1 = m2; y2 = m2; break;
+                }
+                if (a.quat && !(u == 1 && sameFrames)) {
+                    int i0 = b - q.srcBack, i1 = b + q.trgtNext;
+                    if (i0 < 0) i0 += a.nY;
+                    if (i1 >= a.nY) i1 -= a.nY;
+                    i1 -= q.trgtBack;
+                    if (i1 < 0) i1 += a.nY;
+                    so3 = so3_distance(ldg_quat(a.quat + ((long long)i0 * a.quatEX + q.src)),
+                                       ldg_quat(a.quat + ((long long)i1 * a.quatEX + q.trgt)));
+                    rl = robust_loss(a, so3);
+                }
+                if (!(u == 1 && sameFd)) fd = __ldg(a.FD + (long long)q.x2 * a.nvy + y2);
+                double li = 0.0;
+                if (needLi) {  // line_integral's sum, in its order
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) {
+                        const double dy = __ldg(a.VY + 3 * y0 + j) - __ldg(a.VY + 3 * y1 + j);
+                        li = li + dy * dy;
+                        li = li + q.dxx[j];
+                    }
+                    li = sqrt(li);
+                }
+                const bool degenerate = (y2 == y1 || q.x2 == q.x1);
+                double c0 = 0, c1 = 0;
+                if (cm == VANILLA && tm == VANILLA) {
+                    c0 = rl + fd;
+                } else if (cm == VANILLA && tm == LENGTH) {
+                    c0 = rl + fd;
+                    c1 = li;
+                } else if (cm == LENGTH && tm == VANILLA) {
+                    c0 = li;
+                } else if (cm == VANILLA && tm == PENALISE_DEGENERATE) {
+                    c0 = rl + fd;
+                    c1 = degenerate ? 0.1 : 1;
+                } else if (cm == PENALISE_DEGENERATE && tm == VANILLA) {
+                    c0 = degenerate ? 0.1 : 1;
+                } else if (cm == FEATURE && tm == SO3_PLAIN) {
+                    c0 = fd;
+                    c1 = fmax(0.0, twoPi - so3);
+                } else if (cm == FEATURE && tm == SO3_ROBUST) {
+                    c0 = fd;
+                    c1 = fmax(0.0, a.maxSO3 - rl);
+                } else if (cm == SO3_ROBUST && tm == FEATURE) {
+                    c0 = rl;
+                    c1 = fmax(0.0, a.maxFd - fd);
+                } else {  // SO3_PLAIN, FEATURE
+                    c0 = so3;
+                    c1 = fmax(0.0, a.maxFd - fd);
+                }
+                a.out0[idx] = c0;
+                if (a.out1) a.out1[idx] = c1;
+                if (a.hist0) {
+                    count_top_digit(topSh, r0, c0);
+                    if (a.hist1) count_top_digit(topSh + kTopBins, r1, c1);
+                }
             }
         }
     }
