@@ -35,6 +35,26 @@ class BranchHeap {
         up(slot);
     }
 
+    // push(value, key) for every key in order, into an empty heap: equal values
+    // pass each other, so every key takes the root and moves its path's keys
+    // down by one.
+    void fill(double value, const std::vector<int>& keys) {
+        std::vector<int> heap(keys.size());
+        long n = 0;
+        for (const int key : keys) {
+            if (key < 0 || key >= cap_ || at_[(size_t)key] >= 0 || n == cap_) continue;
+            long slot = n++;
+            at_[(size_t)key] = 0;
+            for (; slot > 0; slot = (slot - 1) / 2) heap[(size_t)slot] = heap[(size_t)((slot - 1) / 2)];
+            heap[0] = key;
+        }
+        for (long i = 0; i < n; ++i) {
+            item_[(size_t)i] = {value, heap[(size_t)i]};
+            at_[(size_t)heap[(size_t)i]] = i;
+        }
+        count_ = n;
+    }
+
     bool decrease(long key, double value) {
         if (key < 0 || key >= cap_) return false;
         const long slot = at_[key];

@@ -1773,38 +1773,47 @@ void Graph::solve_min_cost(int K) {
     // product_space.cpp:122-131), else the in-edge sets of layer 0
     // (dijkstra_solver.cpp:93-94).  Entries are used as edge ids
     // (SRCIds(e)), exactly as the reference does (dijkstra_solver.cpp:137-139).
-    std::vector<std::vector<long>> bg;
-    const bool haveBranchGraph = conj || prune;
-    if (haveBranchGraph) {
-        std::vector<std::set<long>> sets((size_t)n);
-        if (!conj) {
-            for (int64_t j = 0; j < nex; ++j) sets[(size_t)EX[2 * j]].insert(EX[2 * j + 1]);
-        } else {
-            std::vector<std::vector<int>> out((size_t)T.nvx);
-            for (int64_t e = 0; e < nex; ++e) out[(size_t)EX[2 * e]].push_back((int)e);
-            const long nE = (long)nex;
-            for (long j = 0; j < nE; ++j) {
-                sets[(size_t)j].insert(j + nE);
-                if (!prune) {
-                    sets[(size_t)(j + nE)].insert(j + 2 * nE);
-                    sets[(size_t)(j + 2 * nE)].insert(j);
-                } else {
-                    sets[(size_t)(j + nE)].insert(j);
-                }
-                for (int e : out[(size_t)EX[2 * j]]) {
-                    sets[(size_t)j].insert(e);
-                    sets[(size_t)(j + nE)].insert(e + nE);
-                    if (!prune) sets[(size_t)(j + 2 * nE)].insert(e + 2 * nE);
-                }
-            }
-        }
-        bg.resize((size_t)n);
-        for (int v = 0; v < n; ++v) bg[(size_t)v].assign(sets[(size_t)v].begin(), sets[(size_t)v].end());
+    // Of a conjugate graph it is implied by the out-edges of the X vertices
+    // (an edge's lists hold its tail's, shifted to the node's kind, and the
+    // next kind of the edge itself), so only those are stored.
+    std::vector<int> bgPtr, bgIds;
+    auto csr = [&](int64_t keys, int64_t count, auto&& key, auto&& id) {
+        bgPtr.assign((size_t)keys + 1, 0);
+        for (int64_t i = 0; i < count; ++i)
+            if (key(i) >= 0) ++bgPtr[(size_t)key(i) + 1];
+        for (int64_t v = 0; v < keys; ++v) bgPtr[(size_t)v + 1] += bgPtr[(size_t)v];
+        bgIds.resize((size_t)bgPtr[(size_t)keys]);
+        std::vector<int> at(bgPtr.begin(), bgPtr.end() - 1);
+        for (int64_t i = 0; i < count; ++i)
+            if (key(i) >= 0) bgIds[(size_t)at[(size_t)key(i)]++] = (int)id(i);
+    };
+    if (conj) {
+        csr(T.nvx, nex, [&](int64_t e) { return EX[(size_t)(2 * e)]; }, [](int64_t e) { return e; });
+    } else if (prune) {
+        csr(n, nex, [&](int64_t j) { return EX[(size_t)(2 * j)]; }, [&](int64_t j) { return EX[(size_t)(2 * j + 1)]; });
+        for (int v = 0; v < n; ++v)
+            std::sort(bgIds.begin() + bgPtr[(size_t)v], bgIds.begin() + bgPtr[(size_t)v + 1]);
     } else {
-        bg.assign((size_t)n, std::vector<long>{-1});
-        for (int64_t t = 0; t < T.eBlock; ++t)
-            if (!T.eNext[(size_t)t]) bg[(size_t)T.eTrgt[(size_t)t]].push_back((long)t);
+        csr(n, T.eBlock, [&](int64_t t) { return T.eNext[(size_t)t] ? -1 : T.eTrgt[(size_t)t]; },
+            [](int64_t t) { return t; });
     }
+    // f(e) for every entry of `node` in ascending order (one that is listed
+    // twice changes nothing the second time).
+    auto for_branch_edges = [&](int node, auto&& f) {
+        if (!conj) {
+            for (int q = bgPtr[(size_t)node]; q < bgPtr[(size_t)node + 1]; ++q) f((long)bgIds[(size_t)q]);
+            return;
+        }
+        const long nE = (long)nex;
+        const int kind = (int)(node / nE);
+        const long j = node - kind * nE;
+        if (kind == 2 && prune) return;
+        if (kind == 2 || (kind == 1 && prune)) f(j);
+        const int tail = EX[(size_t)(2 * j)];
+        for (int q = bgPtr[(size_t)tail]; q < bgPtr[(size_t)tail + 1]; ++q) f(bgIds[(size_t)q] + kind * nE);
+        if (kind == 0) f(j + nE);
+        if (kind == 1 && !prune) f(j + 2 * nE);
+    };
     // SRCIds(e) of an edge id (block * eBlock + offset).
     auto src_of = [&](long e) -> long {
         if (e < 0) return -1;
@@ -1878,49 +1887,48 @@ void Graph::solve_min_cost(int K) {
         std::vector<double> lb((size_t)n);
         d2h(lb.data(), wLb.p, sizeof(double) * n);
         PGC_CUDA(sync_stream());
-        lowerBounds.clear();
-        for (int v = 0; v < n; ++v)
-            if (branchOf[(size_t)v] == branchId) lowerBounds.push_back({lb[(size_t)v], v});
-        std::sort(lowerBounds.begin(), lowerBounds.end());
-        std::vector<double> mark((size_t)n, -1.0);
+        std::vector<unsigned char> mark((size_t)n, 0);
         BranchHeap h(n);
-        for (int i = 0; i < n; ++i) {
-            mark[(size_t)i] = -1;
-            if (i == branchingSrcNode || i == branchingTargetNode) { mark[(size_t)i] = 1; continue; }
-            if (branchOf[(size_t)i] == branchId) h.push(std::numeric_limits<double>::infinity(), i);
+        std::vector<int> members;
+        lowerBounds.clear();
+        for (int v = 0; v < n; ++v) {
+            if (v == branchingSrcNode || v == branchingTargetNode) {
+                mark[(size_t)v] = 1;
+                continue;
+            }
+            if (branchOf[(size_t)v] != branchId) continue;
+            members.push_back(v);
+            lowerBounds.push_back({lb[(size_t)v], v});
         }
+        h.fill(std::numeric_limits<double>::infinity(), members);
         h.push(0.0, branchingSrcNode);
         h.push(0.0, branchingTargetNode);
         if (branchingTargetNode >= 0 && branchingTargetNode < n) branchOf[(size_t)branchingTargetNode] = newId;
-        int counter = 0;
-        for (const auto& e : lowerBounds) {
-            const int v = e.second;
-            if (v == branchingSrcNode || v == branchingTargetNode) continue;
-            if (branchOf[(size_t)v] != branchId) continue;
-            if (counter > std::max(1, numNodesInBranch / 4)) {
-                h.push(0.1, v);
-                branchOf[(size_t)v] = newId;
-            }
-            ++counter;
+        // The members past the first quarter in the order of (lower bound,
+        // node) join the new branch.  (The reference also pushes them onto the
+        // heap, which holds them already and ignores that.)
+        const size_t keep = (size_t)std::max(1, numNodesInBranch / 4) + 1;
+        if (lowerBounds.size() > keep) {
+            std::nth_element(lowerBounds.begin(), lowerBounds.begin() + (long)keep, lowerBounds.end());
+            for (size_t i = keep; i < lowerBounds.size(); ++i) branchOf[(size_t)lowerBounds[i].second] = newId;
         }
         while (!h.isEmpty()) {
             const auto cur = h.pop();
+            // every key left is infinite too: no step from there is shorter
+            if (std::isinf(cur.first)) break;
             const int node = (int)cur.second;
             const float nodeCost = (float)cur.first;
-            mark[(size_t)node] = 1.0;
-            for (long e : bg[(size_t)node]) {
-                if (e == -1) continue;
-                const long s = haveBranchGraph ? src_of(e) : src_of(e);
-                if (s < 0 || s >= n) continue;
-                if (mark[(size_t)s] < 0) {
-                    const float oldV = (float)h.peakKey(s);
-                    const float newV = nodeCost + 1.0f;
-                    if (newV < oldV) {
-                        h.decrease(s, newV);
-                        branchOf[(size_t)s] = branchOf[(size_t)node];
-                    }
+            mark[(size_t)node] = 1;
+            for_branch_edges(node, [&](long e) {
+                const long s = src_of(e);
+                if (s < 0 || s >= n || mark[(size_t)s]) return;
+                const float oldV = (float)h.peakKey(s);
+                const float newV = nodeCost + 1.0f;
+                if (newV < oldV) {
+                    h.decrease(s, newV);
+                    branchOf[(size_t)s] = branchOf[(size_t)node];
                 }
-            }
+            });
         }
         branchingSrcNode = -1;
         branchingTargetNode = -1;
