@@ -142,17 +142,14 @@ struct LocalStreams {
     unsigned ls, c, t;            // byte offsets of the lane's entries: source index, cost, time
     const CT* gc;
     const char* gt;
-    __device__ __forceinline__ double weight(int r, double lam, double lt) const {
-        double x = lt;
-        if constexpr (TK == 1) {
-            const float f = STAGED ? local_at<float>(t)[r * 32] : reinterpret_cast<const float*>(gt)[r * 32];
-            x = __dmul_rn(lam, (double)f);
-        }
-        if constexpr (TK == 2) {
-            const double f = STAGED ? local_at<double>(t)[r * 32] : reinterpret_cast<const double*>(gt)[r * 32];
-            x = __dmul_rn(lam, f);
-        }
-        return __dsub_rn((double)(STAGED ? local_at<CT>(c)[r * 32] : gc[r * 32]), x);
+    using Time = std::conditional_t<TK == 2, double, float>;
+    __device__ __forceinline__ CT cost(int r) const { return STAGED ? local_at<CT>(c)[r * 32] : gc[r * 32]; }
+    __device__ __forceinline__ Time time(int r) const {
+        if constexpr (TK == 0) return Time(0);
+        else return STAGED ? local_at<Time>(t)[r * 32] : reinterpret_cast<const Time*>(gt)[r * 32];
+    }
+    static __device__ __forceinline__ double weight(CT c, Time t, double lam, double lt) {
+        return __dsub_rn((double)c, TK == 0 ? lt : __dmul_rn(lam, (double)t));
     }
     __device__ __forceinline__ void advance(int rows) {
         constexpr int timeBytes = TK == 1 ? 4 : TK == 2 ? 8 : 0;
@@ -170,8 +167,16 @@ struct LocalStreams {
 template <class CT, int TK, bool STAGED, int KD, int NK, int CH, int NR>
 __device__ __forceinline__ void local_batch(const LocalStreams<CT, TK, STAGED>& q, unsigned sval, double lam, double lt,
                                             int row8, double (&thr)[CH * NK], int (&win)[CH * NK]) {
+    using Streams = LocalStreams<CT, TK, STAGED>;
     unsigned si[NR];
-    double w[NR], d[NR][NK];
+    double d[NR][NK];
+    CT cost[NR];
+    typename Streams::Time time[NR];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+        cost[r] = q.cost(r);
+        time[r] = q.time(r);
+    }
 #pragma unroll
     for (int r = 0; r < NR; ++r) si[r] = sval + (unsigned)local_at<unsigned short>(q.ls)[r * 32] * (KD * 8);
 #pragma unroll
@@ -188,18 +193,18 @@ __device__ __forceinline__ void local_batch(const LocalStreams<CT, TK, STAGED>& 
         }
     }
 #pragma unroll
-    for (int r = 0; r < NR; ++r) w[r] = q.weight(r, lam, lt);
-#pragma unroll
-    for (int r = 0; r < NR; ++r)
+    for (int r = 0; r < NR; ++r) {
+        const double w = Streams::weight(cost[r], time[r], lam, lt);
 #pragma unroll
         for (int kk = 0; kk < NK; ++kk) {
-            const double cand = __dadd_rn(d[r][kk], w[r]);
+            const double cand = __dadd_rn(d[r][kk], w);
             const int c = (r % CH) * NK + kk;
             if (cand < thr[c]) {
                 thr[c] = cand;
                 win[c] = row8 + (r * 8 + kk);
             }
         }
+    }
 }
 
 template <class CT, int TK, bool STAGED, int KD, int NK, int CH, int NR>

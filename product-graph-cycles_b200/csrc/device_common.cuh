@@ -248,12 +248,13 @@ struct LookupArgs {
 // bound (cost_time_ratio_solver.cpp:652-707), the Lawler iterations
 // (:558-635) and their cycle evaluations (computeRatioForCycle, :88-133) --
 // as long as the first branch's cycle does not wrap; otherwise the host
-// finishes the solve with branch and bound.
+// goes on from that cycle with branch and bound.
 enum PairStatus : int {
     PAIR_PENDING = 0,
     PAIR_DONE = 1,       // result written
     PAIR_NAN = 2,        // the reference's (true, NaN, no rows) result
-    PAIR_HOST = 3,       // the solve needs branch and bound (or a longer cycle record): finish on the host
+    PAIR_HOST = 3,       // the solve needs the host from the start (a longer cycle record, no finite bound)
+    PAIR_WRAPS = 4,      // the first branch's cycle wraps: the host goes on from it with branch and bound
     PAIR_ERR_UB = -1,    // no closed path through the upper-bound start node
     PAIR_ERR_EDGE = -2,  // a cycle edge was not found in the product graph
     PAIR_ERR_BF = -3,    // a Bellman-Ford call ended in an error status (in bfStatus)
@@ -284,6 +285,8 @@ struct PairJob {
     int rec;
     double adjT;           // time sum of the returned cycle (the adjoint's T)
     double ratio;          // its ratio C / T in double (the adjoint's lambda*)
+    double bound;          // the initial upper bound
+    double lambda;         // Lawler's last ratio in the first branch
     long long cycles;      // SM clock cycles the CTA spent on the graph
     long long bfCalls, sweeps, lawlerIters, candidates, fallbackWalks;
 };
@@ -299,14 +302,15 @@ constexpr long long kWalkRoundLoads = 4096;
 constexpr int kBfThreads = 640;
 // Source values a lane gathers before folding them (one batch of rows).
 constexpr int kGather = 20;
-// Relaxing threads of a batched-solve CTA (one staging warp comes on top) and
-// the CTAs an SM holds: one, so that a graph's local tables and step buffers
-// get the SM's shared memory.
+// Threads of a batched-solve CTA, one of its warps the staging warp.  One CTA
+// takes an SM, so that a graph's local tables and step buffers get its shared
+// memory; 20 warps, five to a scheduler, leave 96 registers each, 21 only 80.
 constexpr int kBatchThreads = 640;
 // Capacity of a batched solve's cycle records (edges); a longer cycle hands
 // the graph back to the host.
 constexpr long long kBatchCycleCap = 1LL << 16;
-constexpr int kBatchBlocksPerSm = 1;
+// Shared memory a launch leaves to the batched kernel's static variables.
+constexpr int kBatchStaticSmem = 5120;
 // Rows of one gather batch when every row has nk source depths (nk > 0).
 __host__ __device__ constexpr int bf_rows_per_batch(int nk) {
     return kGather / nk < 1 ? 1 : kGather / nk > 8 ? 8 : kGather / nk;

@@ -44,6 +44,7 @@
 #include <mutex>
 #include <set>
 #include <tuple>
+#include <type_traits>
 
 #include "device_common.cuh"
 
@@ -633,6 +634,7 @@ __device__ int lap_walk(const BfParams& p, int x0, long long limit, int* v0, lon
     int hare = __ldcg(P + x0);
     long long guard = 0;
     const long long guardMax = 4LL * (p.n + 2);
+    const int n = p.n;
     while (hare != tort) {
         if (hare < 0) return hare == kLapEnd ? 2 : 3;
         if (power == lam) { tort = hare; power <<= 1; lam = 0; }
@@ -647,7 +649,7 @@ __device__ int lap_walk(const BfParams& p, int x0, long long limit, int* v0, lon
     while (tort != hare) {
         tort = __ldcg(P + tort);
         hare = __ldcg(P + hare);
-        if (++mu > p.n + 1) return 3;
+        if (++mu > n + 1) return 3;
     }
     long long S = 0;
     int x = x0;
@@ -809,14 +811,19 @@ __device__ int lap_cycle_list(const BfParams& p, int v0, int* nodes, long long* 
 // last step, which must reach xNext; otherwise (or when a predecessor leaves
 // the node range) it returns non-zero and the serial walk decides.
 __device__ int walk_lap(const BfParams& p, int x, int xNext, long long off, long long len) {
-    const long long total = (long long)p.n * (p.nY + 1) * p.K;
+    const int n = p.n, K = p.K, total = (int)((long long)n * (p.nY + 1) * K);
+    const int* pred = p.pred;
+    int* out = p.cycleBuf + off;
     int pr = x;
-    for (long long s = 0; s < len; ++s) {
-        pr = __ldcg(p.pred + pr);
+    for (int s = 0, end = (int)len; s < end; ++s) {
+        pr = __ldcg(pred + pr);
         if (pr < 0 || pr >= total) return 1;
-        if (pr < p.n && s + 1 < len) return 2;
-        p.cycleBuf[off + s] = original_index(p.n, p.K, pr);
+        if (pr < n && s + 1 < end) return 2;
+        out[s] = pr;
     }
+    // the chain of loads first, then the node ids: the divisions would
+    // lengthen every link
+    for (int s = 0; s < (int)len; ++s) out[s] = original_index(n, K, out[s]);
     return pr == xNext ? 0 : 2;
 }
 
@@ -825,20 +832,26 @@ __device__ int walk_lap(const BfParams& p, int x, int xNext, long long off, long
 __device__ int extract_ub_path(const BfParams& p, int start) {
     const int n = p.n, K = p.K;
     const long long total = (long long)n * (p.nY + 1) * K;
-    const long long maxLength = (long long)p.nY * K;
+    const long long maxLength = (long long)p.nY * K, cap = p.cycleCap;
     const long long firstV = start + (long long)n * p.nY * K;
+    const int* pred = p.pred;
+    int* out = p.cycleBuf;
+    // the chain of loads first, then the node ids: the divisions would
+    // lengthen every link
     int len = 0;
-    p.cycleBuf[len++] = original_index(n, K, (int)firstV);
-    int pr = __ldcg(p.pred + firstV);
-    p.cycleBuf[len++] = (pr >= 0 && pr < total) ? original_index(n, K, pr) : -1;
+    out[len++] = (int)firstV;
+    int pr = __ldcg(pred + firstV);
+    out[len++] = (pr >= 0 && pr < total) ? pr : -1;
     for (long long kk = maxLength - 1; kk > 0; --kk) {
         if (pr == -1) break;
         if (pr < 0 || pr >= total) return BF_ERR_WALK;
-        pr = __ldcg(p.pred + pr);
-        if (len >= p.cycleCap) return BF_ERR_CYCLE_CAP;
-        p.cycleBuf[len++] = (pr >= 0 && pr < total) ? original_index(n, K, pr) : -1;
+        pr = __ldcg(pred + pr);
+        if (len >= cap) return BF_ERR_CYCLE_CAP;
+        out[len++] = (pr >= 0 && pr < total) ? pr : -1;
         if (pr == start) break;
     }
+    for (int i = 0; i < len; ++i)
+        if (out[i] >= 0) out[i] = original_index(n, K, out[i]);
     p.ctl->cycleLen = len;
     return BF_UB_DONE;
 }
@@ -1400,7 +1413,7 @@ __global__ void __launch_bounds__(kBfThreads, 1) bf_kernel(BfParams p) {
 
 // The same on per-CTA local tables (bf_local.cuh).
 template <class CT, int TK>
-__global__ void __launch_bounds__(kBfThreads + 32, 1) bf_local_kernel(const __grid_constant__ BfParams p) {
+__global__ void __launch_bounds__(kBfThreads, 1) bf_local_kernel(const __grid_constant__ BfParams p) {
     const Team t{(int)blockIdx.x, (int)gridDim.x, &p.ctl->barCount, &p.ctl->barGen, &p.ctl->error, p.spinLimit};
     bf_body<CT, TK, false, 1>(p, t, nullptr);
 }
@@ -1590,23 +1603,42 @@ __device__ __forceinline__ int round_to_int_x86(double x) {
 __device__ __forceinline__ double via_float(double x) { return (double)__double2float_rn(x); }
 
 struct CycleSums {
-    double ratio, wsum;
+    double ratio, wsum, time;
 };
 
-// computeRatioForCycle's sums over a stored cycle record, one thread, in the
-// cycle's order: C += c, T += t, W += c - lambda * t, each a rounded double
-// operation.
+// computeRatioForCycle's sums over a stored cycle record in the cycle's order:
+// C += c, T += t, W += c - lambda * t, each a rounded double operation.  Every
+// CTA calls it with all its threads, which bring the record into shared memory
+// in parts for the one that adds (its own loads, one after the other, were 700
+// cycles an edge).  The result is every thread's.
 __device__ CycleSums record_sums(const PairJob& J, int rec, int m, double lambda) {
+    constexpr int kPart = 128;
+    __shared__ double sc[kPart], st[kPart];
+    __shared__ CycleSums out;
     const double* c = J.recC[rec];
     const double* t = J.recT[rec];
     double C = 0, T = 0, W = 0;
-    for (int i = 0; i < m; ++i) {
-        const double ci = __ldcg(c + i), ti = __ldcg(t + i);
-        C = __dadd_rn(C, ci);
-        T = __dadd_rn(T, ti);
-        W = __dadd_rn(W, __dsub_rn(ci, __dmul_rn(lambda, ti)));
+    for (int i0 = 0; i0 < m; i0 += kPart) {
+        const int n = min(kPart, m - i0);
+        for (int i = (int)threadIdx.x; i < 2 * n; i += blockDim.x) {
+            if (i < n) sc[i] = __ldcg(c + i0 + i);
+            else st[i - n] = __ldcg(t + i0 + i - n);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int i = 0; i < n; ++i) {
+                const double ci = sc[i], ti = st[i];
+                C = __dadd_rn(C, ci);
+                T = __dadd_rn(T, ti);
+                W = __dadd_rn(W, __dsub_rn(ci, __dmul_rn(lambda, ti)));
+            }
+        __syncthreads();
     }
-    return {__ddiv_rn(C, T), W};
+    if (threadIdx.x == 0) out = CycleSums{__ddiv_rn(C, T), W, T};
+    __syncthreads();
+    const CycleSums r = out;
+    __syncthreads();
+    return r;
 }
 
 // The CTAs that solve one graph together: `all` is the whole team, with
@@ -1658,15 +1690,12 @@ __device__ int record_cycle(const PairJob& J, const BfParams& P, const Team& t, 
     return anyMissing ? -1 : m;
 }
 
-// Lawler's outcome of one Bellman-Ford call (the host driver's bellman_ford).
-enum Outcome { OUT_FOUND = 0, OUT_NONE = 1, OUT_ZERO = 2 };
-
 template <class CT, int TK>
 __device__ __noinline__ void bf_call(const BfParams& P, const Team& t) {
     bf_body<CT, TK, false>(P, t, reinterpret_cast<char*>(smemRaw));
 }
 template <class CT, int TK>
-__device__ __noinline__ void bf_local_call(const BfParams& P, const Team& t) {
+__device__ __forceinline__ void bf_local_call(const BfParams& P, const Team& t) {
     bf_body<CT, TK, false, 2>(P, t, nullptr);
 }
 
@@ -1674,7 +1703,7 @@ __device__ __noinline__ void bf_local_call(const BfParams& P, const Team& t) {
 // the Bellman-Ford CTAs run it, and every CTA reads its verdict after the
 // closing barrier.  False when a team barrier ran out.
 template <class CT, int TK>
-__device__ bool team_bf_call(PairJob& J, const BfParams& P, const SolveTeam& S, bool resetError) {
+__device__ __forceinline__ bool team_bf_call(PairJob& J, const BfParams& P, const SolveTeam& S, bool resetError) {
     if (S.lead()) {
         P.ctl->status = BF_RUNNING;
         if (resetError) P.ctl->error = 0;
@@ -1698,9 +1727,7 @@ __device__ bool team_bf_call(PairJob& J, const BfParams& P, const SolveTeam& S, 
 // one thread of every CTA, in the same order, so every CTA takes the same
 // branches; only the lead writes the job's outputs.
 template <class CT, int TK>
-__device__ void pair_solve(PairJob& J, BfParams& P, const SolveTeam& S) {
-    __shared__ int sState[4];        // [1] the bound search gave up, [3] edges of the last record
-    __shared__ double sRatio;
+__device__ __forceinline__ void pair_solve(PairJob& J, BfParams& P, const SolveTeam& S) {
     const Team& t = S.all;
     const bool lead = S.lead();
     const int n = P.n;
@@ -1758,84 +1785,68 @@ __device__ void pair_solve(PairJob& J, BfParams& P, const SolveTeam& S) {
     }
     const int startV = best.i == 0x7fffffff ? 0 : best.i;
     for (long long v = t.thread(); v < n; v += t.nthreads()) J.branchOf[v] = v == startV ? 0 : 1;
-    if (threadIdx.x == 0) {
-        P.mode = 1;
-        P.branchId = 0;
-        P.lambda = 10;
-        P.ub = ubInf;
-    }
-    if (!team_bf_call<CT, TK>(J, P, S, true)) PGC_TEAM_FAIL();
-    if (*(volatile int*)&ctl->error) PGC_TEAM_FAIL();
-    {
-        const int st = *(volatile int*)&ctl->status;
-        if (st == BF_LAYER_UNREACHED) {  // the empty cycle's 0/0 bound: (true, NaN, no rows)
-            if (lead) J.status = PAIR_NAN;
-            return;
-        }
-        if (st != BF_UB_DONE) {
-            if (lead) {
-                J.status = st < 0 ? PAIR_ERR_BF : PAIR_ERR_UB;
-                J.bfStatus = st;
-            }
-            return;
-        }
-    }
-    int neg = 0;
-    {
-        const int m = record_cycle(J, P, t, neg, *(volatile int*)&ctl->cycleLen, false);
-        if (m == -3) PGC_TEAM_FAIL();
-        if (m < 0) {
-            if (lead) J.status = m == -2 ? PAIR_HOST : PAIR_ERR_EDGE;
-            return;
-        }
-        if (threadIdx.x == 0) {
-            sState[3] = m;
-            double lambda = 10;
-            CycleSums ev = record_sums(J, neg, m, lambda);
-            double cycleCost = via_float(ev.wsum);
-            int guard = 0, bad = 0;
-            while (cycleCost > 0 || isnan(cycleCost)) {
-                if (++guard > 4000) {
-                    bad = 1;
-                    break;
-                }
-                lambda += lambda;
-                ev = record_sums(J, neg, m, lambda);
-                cycleCost = via_float(ev.wsum);
-            }
-            sRatio = via_float(ev.ratio);
-            sState[1] = bad;
-        }
-        __syncthreads();
-        if (sState[1]) {
-            if (lead) J.status = PAIR_ERR_GUARD;
-            return;
-        }
-    }
-    // A NaN or infinite bound: the host's branch-and-bound path (the heap
-    // comparison that ends the first branch does not hold then).
-    if (!(sRatio < (double)__int_as_float(0x7f800000))) {
-        if (lead) J.status = PAIR_HOST;
-        return;
-    }
-
-    // ---- the first branch: every node starts (cost_time_ratio_solver.cpp:794-829) ----
-    for (long long v = t.thread(); v < n; v += t.nthreads()) J.branchOf[v] = 0;
-    double currentRatio = sRatio;  // every thread keeps the same copy
-    double oldRatio = currentRatio;
-    int negEdges = sState[3];
+    // The first call is the bound's sweep; the others are Lawler's in the first
+    // branch, where every node starts (cost_time_ratio_solver.cpp:794-829).  One
+    // call site: the step loop is then a callee of the kernel itself.  Every
+    // thread of every CTA keeps the same copies and takes the same turns.
+    int neg = 0, negEdges = 0;
+    double bound = 0, currentRatio = 10, oldRatio = 0;
+    CycleSums sums{};  // of the current negative cycle
+    bool search = true;
     for (int i = 0;;) {
         if (threadIdx.x == 0) {
-            P.mode = 0;
+            P.mode = search ? 1 : 0;
             P.branchId = 0;
             P.lambda = currentRatio;
             P.ub = ubInf;
         }
-        if (!team_bf_call<CT, TK>(J, P, S, false)) PGC_TEAM_FAIL();
-        if (lead) J.lawlerIters++;
+        if (!team_bf_call<CT, TK>(J, P, S, search)) PGC_TEAM_FAIL();
+        if (lead && !search) J.lawlerIters++;
         if (*(volatile int*)&ctl->error) PGC_TEAM_FAIL();
         const int st = *(volatile int*)&ctl->status;
-        int outcome;
+        if (search) {
+            if (st == BF_LAYER_UNREACHED) {  // the empty cycle's 0/0 bound: (true, NaN, no rows)
+                if (lead) J.status = PAIR_NAN;
+                return;
+            }
+            if (st != BF_UB_DONE) {
+                if (lead) {
+                    J.status = st < 0 ? PAIR_ERR_BF : PAIR_ERR_UB;
+                    J.bfStatus = st;
+                }
+                return;
+            }
+            const int m = record_cycle(J, P, t, neg, *(volatile int*)&ctl->cycleLen, false);
+            if (m == -3) PGC_TEAM_FAIL();
+            if (m < 0) {
+                if (lead) J.status = m == -2 ? PAIR_HOST : PAIR_ERR_EDGE;
+                return;
+            }
+            negEdges = m;
+            double lambda = 10;
+            CycleSums ev = record_sums(J, neg, m, lambda);
+            for (int guard = 0; via_float(ev.wsum) > 0 || isnan(via_float(ev.wsum));) {
+                if (++guard > 4000) {
+                    if (lead) J.status = PAIR_ERR_GUARD;
+                    return;
+                }
+                lambda += lambda;
+                ev = record_sums(J, neg, m, lambda);
+            }
+            bound = via_float(ev.ratio);
+            // A NaN or infinite bound: the host's branch-and-bound path (the
+            // heap comparison that ends the first branch does not hold then).
+            if (!(bound < (double)__int_as_float(0x7f800000))) {
+                if (lead) J.status = PAIR_HOST;
+                return;
+            }
+            for (long long v = t.thread(); v < n; v += t.nthreads()) J.branchOf[v] = 0;
+            currentRatio = oldRatio = bound;
+            search = false;
+            continue;
+        }
+        // the call's outcome is a new negative cycle, or the end: a cycle that
+        // is not negative and an old one that is zero by now both end Lawler
         if (st == BF_FOUND_CYCLE) {
             const int cand = neg ^ 1;
             const int m = record_cycle(J, P, t, cand, *(volatile int*)&ctl->cycleLen, true);
@@ -1844,29 +1855,13 @@ __device__ void pair_solve(PairJob& J, BfParams& P, const SolveTeam& S) {
                 if (lead) J.status = m == -2 ? PAIR_HOST : PAIR_ERR_EDGE;
                 return;
             }
-            if (threadIdx.x == 0) {
-                const int integral = round_to_int_x86(record_sums(J, cand, m, currentRatio).wsum);
-                int o;
-                if (integral < 0) o = OUT_FOUND;
-                else if (integral == 0) o = OUT_NONE;
-                else o = round_to_int_x86(record_sums(J, neg, negEdges, currentRatio).wsum) == 0 ? OUT_ZERO : OUT_NONE;
-                sState[0] = o;
-                sState[3] = m;
-            }
-            __syncthreads();
-            outcome = sState[0];
-            if (outcome == OUT_FOUND) {
-                neg = cand;
-                negEdges = sState[3];
-            }
+            const CycleSums ev = record_sums(J, cand, m, currentRatio);
+            if (round_to_int_x86(ev.wsum) >= 0) break;
+            neg = cand;
+            negEdges = m;
+            sums = ev;
         } else if (st == BF_LAYER_UNREACHED || st == BF_WRAP_NO_IMPROVE || st == BF_MAX_SWEEPS) {
-            if (threadIdx.x == 0)
-                sState[0] = st != BF_MAX_SWEEPS &&
-                                    round_to_int_x86(record_sums(J, neg, negEdges, currentRatio).wsum) == 0
-                                ? OUT_ZERO
-                                : OUT_NONE;
-            __syncthreads();
-            outcome = sState[0];
+            break;
         } else {
             if (lead) {
                 J.status = PAIR_ERR_BF;
@@ -1874,43 +1869,43 @@ __device__ void pair_solve(PairJob& J, BfParams& P, const SolveTeam& S) {
             }
             return;
         }
-        if (outcome != OUT_FOUND) break;
         // lawlerSoubroutine's update and stopping rules (:584-597)
-        if (threadIdx.x == 0) sRatio = record_sums(J, neg, negEdges, currentRatio).ratio;
-        __syncthreads();
-        currentRatio = sRatio;
+        currentRatio = sums.ratio;
         if (fabs(oldRatio - currentRatio) < tolerance) break;
         if (currentRatio - tolerance > oldRatio) break;
         oldRatio = currentRatio;
         if (i > 1000) break;
         ++i;
     }
+    const CycleSums fin = record_sums(J, neg, negEdges, currentRatio);
     // passes of the cycle through layer 0 (:606-634): more than one, and the
     // branch and bound splits the branch -- the host's part
-    if (lead) {
+    if (t.cta != 0) return;
+    __shared__ int sWraps;
+    if (threadIdx.x == 0) sWraps = 0;
+    __syncthreads();
+    {
+        // runs of nodes outside layer 0
         const int* nodes = J.recNodes[neg];
-        int wraps = 0;
-        bool left = false;
-        for (int i = 0; i <= negEdges; ++i) {
-            const int vtx = __ldcg(nodes + i);
-            if (left && vtx < n) left = false;
-            if (vtx >= n && !left) {
-                ++wraps;
-                left = true;
-            }
-        }
+        int runs = 0;
+        for (int i = (int)threadIdx.x; i <= negEdges; i += blockDim.x)
+            if (__ldcg(nodes + i) >= n && (i == 0 || __ldcg(nodes + i - 1) < n)) ++runs;
+        if (runs) atomicAdd(&sWraps, runs);
+    }
+    __syncthreads();
+    if (lead) {
+        const int wraps = sWraps;
+        J.nEdges = negEdges;
+        J.rec = neg;
+        J.adjT = fin.time;
+        J.ratio = fin.ratio;
+        J.bound = bound;
+        J.lambda = currentRatio;
         if (wraps > 1 && n > 1) {
-            J.status = PAIR_HOST;
+            J.status = PAIR_WRAPS;
         } else {
-            const CycleSums fin = record_sums(J, neg, negEdges, currentRatio);
-            double T = 0;
-            for (int i = 0; i < negEdges; ++i) T += __ldcg(J.recT[neg] + i);
             J.passes = 1;
             J.objective = __double2float_rn(fin.ratio);
-            J.nEdges = negEdges;
-            J.rec = neg;
-            J.adjT = T;
-            J.ratio = fin.ratio;
             J.status = PAIR_DONE;
         }
     }
@@ -1925,7 +1920,7 @@ __device__ void pair_solve(PairJob& J, BfParams& P, const SolveTeam& S) {
 // With more than one CTA per team the launch is cooperative, so that every
 // CTA of a team is resident.
 template <class CT, int TK>
-__global__ void __launch_bounds__(kBatchThreads + 32, kBatchBlocksPerSm)
+__global__ void __launch_bounds__(kBatchThreads, 1)
     bf_batch_kernel(PairJob* jobs, int count, int* next, unsigned* teamWords, int teamCtas, unsigned spin) {
     __shared__ BfParams P;
     __shared__ int sJob, sCtas;

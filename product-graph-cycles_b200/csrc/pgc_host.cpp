@@ -467,7 +467,7 @@ class Graph {
         const void* time;
         double tconst;
         int blocks, threads;
-        int extraThreads;   // launched on top: the staging warp of teams on local tables
+        int extraThreads;   // launched on top of `threads`
         bool coop;
         bool sharedTables;  // single CTA keeping its DP records in shared memory
         int flagSync;       // neighbour hand-offs between steps (multi-CTA teams)
@@ -498,7 +498,17 @@ class Graph {
     int batchThreads = 0;
     int batchCtas = 1;
     size_t batchSmemCap = 0;
-    void solve_ratio_rescaled(int K);
+    // The first branch's outcome, when the device ran it.
+    struct FirstBranch {
+        double bound, lambda;
+        CycleRec cycle;
+    };
+    void solve_ratio_rescaled(int K, const FirstBranch* first = nullptr);
+    bool solve_ratio_device(int K);
+    void fill_job(const Run& r, PairJob& J);
+    void finish_job(const PairJob& J, int K);
+    DBuf<PairJob> wJob;
+    DBuf<unsigned> wJobWords;  // the team's barrier words, then the queue's counter
     void ensure_workspace(int K, int blocks);
     std::vector<int> cta_cuts(int blocks, int K, int warps) const;
     void upload_cta_slices(const std::vector<int>& cut, int K, int warps);
@@ -892,15 +902,15 @@ Graph::Run Graph::prepare_run(int K, bool ratio) {
             if (teamCap > 0) lb = std::min(lb, teamCap);
         }
         lb = std::max(1, std::min({lb, T.nslices, sms}));
-        // relaxing warps: one per slice of the largest share, at most 20; the
-        // launch adds one that stages the streams
-        r.threads = envThreads ? envThreads
-                               : std::min(kBfThreads, 32 * std::max(2, (active + lb - 1) / lb));
-        if (plan_local(r, lb, smemCap)) {
-            r.extraThreads = 32;
+        // a relaxing warp per slice of the largest share, and the one that
+        // stages the streams
+        r.threads = envThreads ? envThreads : std::min(kBfThreads, 32 * (1 + (active + lb - 1) / lb));
+        if (plan_local(r, lb, (size_t)std::max(0, smemOptin - kBatchStaticSmem))) {
+            r.extraThreads = r.threads == 32 ? 32 : 0;  // a relaxing warp at least
             if (r.blocks > 1) {
                 int perSm = 0;
-                PGC_CUDA(bf_max_coop_blocks(r.costF32, r.timeKind, true, r.threads + 32, r.smemBytes, &perSm));
+                if (ratio) PGC_CUDA(bf_batch_max_blocks(r.costF32, r.timeKind, r.threads + r.extraThreads, r.smemBytes, &perSm));
+                else PGC_CUDA(bf_max_coop_blocks(r.costF32, r.timeKind, true, r.threads + r.extraThreads, r.smemBytes, &perSm));
                 if (perSm < 1) throw Failure(PGC_ERR_CUDA, "the Bellman-Ford kernel cannot be resident with its shared memory");
             }
             r.coop = r.blocks > 1;
@@ -1370,20 +1380,56 @@ RatioEval eval_cycle(const CycleRec& cy, double lambda) {
 void Graph::solve_ratio(int K) {
     ensure_generated();
     stats = Stats();
-    const auto wall0 = std::chrono::steady_clock::now();
     const double scaling = 100000.0;
     // In-place rescale of the generator's costs (cost_time_ratio_solver.cpp:875-882).
     rescale_columns(scaling);
-    solve_ratio_rescaled(K);
-    (void)wall0;
+    if (!solve_ratio_device(K)) solve_ratio_rescaled(K);
+}
+
+// The ratio solve by one launch of the batched solver with this graph alone:
+// its whole team runs the upper bound, the Lawler iterations and the cycle
+// evaluations on the device, where the host-driven solve waits twice per
+// Bellman-Ford call.  False: the graph's team does not run on local tables.
+bool Graph::solve_ratio_device(int K) {
+    const Run r = prepare_run(K, true);
+    if (!r.localKD) return false;
+    reset_predecessors();
+    PairJob J;
+    fill_job(r, J);
+    wJob.alloc(1);
+    wJobWords.alloc(kTeamWordStride + 1);
+    wJobWords.zero(stream);
+    PGC_CUDA(cudaMemcpyAsync(wJob.p, &J, sizeof(PairJob), cudaMemcpyHostToDevice, stream));
+    if (!timeEvents[0]) {
+        PGC_CUDA(cudaEventCreate(&timeEvents[0]));
+        PGC_CUDA(cudaEventCreate(&timeEvents[1]));
+    }
+    PGC_CUDA(cudaEventRecord(timeEvents[0], stream));
+    PGC_CUDA(launch_bf_batch(wJob.p, 1, reinterpret_cast<int*>(wJobWords.p + kTeamWordStride), wJobWords.p, r.blocks,
+                             J.bf.spinLimit, r.costF32, r.timeKind, r.blocks, r.threads + r.extraThreads, r.smemBytes,
+                             stream));
+    PGC_CUDA(cudaEventRecord(timeEvents[1], stream));
+    const long long launches = stats.launches;
+    d2h(&J, wJob.p, sizeof(PairJob));
+    PGC_CUDA(sync_stream());
+    float ms = 0;
+    cudaEventElapsedTime(&ms, timeEvents[0], timeEvents[1]);
+    finish_job(J, K);
+    if (J.status != PAIR_HOST) {
+        stats.deviceMs += ms;
+        stats.launches += launches + 1;
+    }
+    return true;
 }
 
 // The ratio solve after the rescale: the initial upper bound, then branch
 // and bound with Lawler in each branch (cost_time_ratio_solver.cpp:741-864).
-void Graph::solve_ratio_rescaled(int K) {
+// `first`: the bound and the first branch's Lawler are done already; what is
+// left starts from that branch's cycle.
+void Graph::solve_ratio_rescaled(int K, const FirstBranch* first) {
     const double scaling = 100000.0;
     Run r = prepare_run(K, true);
-    reset_predecessors();
+    if (!first) reset_predecessors();
     const int n = T.n;
     const long long nn = numNodes();
     const double tconst = ncols > 1 ? 0.0 : scaling / 2;
@@ -1415,7 +1461,9 @@ void Graph::solve_ratio_rescaled(int K) {
     int numNodesInBranch = 0;
 
     // ---- initial upper bound (cost_time_ratio_solver.cpp:652-707) ----
-    {
+    if (first) {
+        currentRatio = first->bound;
+    } else {
         std::vector<float> mean((size_t)n);
         std::vector<int> cnt((size_t)n);
         if (e64Stale[0])
@@ -1520,7 +1568,12 @@ void Graph::solve_ratio_rescaled(int K) {
         int i = 0;
         const int maxiter = 1000;
         double oldRatio = currentRatio;
-        for (;;) {
+        if (first) {
+            negativeCycle = first->cycle;
+            currentRatio = first->lambda;
+            numNodesInBranch = n;
+        }
+        while (!first) {
             const BfOutcome s = bellman_ford(currentRatio);
             stats.lawlerIters++;
             if (s != BfOutcome::FOUND_NEGATIVE_CYCLE) break;
@@ -1531,6 +1584,7 @@ void Graph::solve_ratio_rescaled(int K) {
             if (i > maxiter) break;
             ++i;
         }
+        first = nullptr;
         lowerBoundOfCurrentBranch = currentRatio;
         int numWraps = 0;
         zeroLayerHits.clear();
@@ -1551,7 +1605,7 @@ void Graph::solve_ratio_rescaled(int K) {
             negativeCycle = validCycles.at(branchId);
             break;
         }
-        stats.branches++;
+        if (!first) stats.branches++;  // the device's first branch is counted
         currentRatio = ratioUpperBound;
         const bool wraps = lawler();
         if (ratioUpperBound < heap.peak() && !wraps) break;
@@ -1592,6 +1646,59 @@ void Graph::solve_ratio_rescaled(int K) {
 // Printed by pgc_solve_batch when PGC_BATCH_PHASES is set.
 std::atomic<long long> g_batchPhaseNs[3];
 
+// The device's description of a ratio solve by the prepared team, its records
+// and its control block.
+void Graph::fill_job(const Run& r, PairJob& J) {
+    // PGC_BATCH_CYCLE_CAP (tests): a smaller record, so that graphs are
+    // handed back to the host
+    const long long capMax = std::min<long long>(kBatchCycleCap, std::max(1, env_int("PGC_BATCH_CYCLE_CAP", (int)kBatchCycleCap)));
+    const int cap = (int)std::min<long long>(numNodes() + 4, capMax);
+    for (int k = 0; k < 2; ++k) {
+        bRecNodes[k].alloc((size_t)cap + 1);
+        bRecEdges[k].alloc((size_t)cap);
+        bRecC[k].alloc((size_t)cap);
+        bRecT[k].alloc((size_t)cap);
+    }
+    J = PairJob{};
+    J.bf = params(r, 0, 0, 0.0, std::numeric_limits<float>::infinity());
+    J.bf.ctaSlice = wCtaSlice.p;
+    J.ctas = r.blocks;
+    J.threads = r.threads;
+    LookupArgs& a = J.lk;
+    a.n = T.n;
+    a.nY = T.nY;
+    a.nodeSlot = dNodeSlot.p;
+    a.numNodes = numNodes();
+    a.eBlock = T.eBlock;
+    a.spInter = dSp[INTER].p;
+    a.spIntra = dSp[INTRA].p;
+    a.srcInter = dSrc[INTER].p;
+    a.srcDummy = dSrcDummy.p ? dSrcDummy.p : dSrc[INTER].p;
+    a.srcIntra = dSrc[INTRA].p;
+    a.tedgeInter = dTedge[INTER].p;
+    a.tedgeIntra = dTedge[INTRA].p;
+    a.interEntries = T.entries[INTER];
+    a.layerStride = T.layerStride();
+    a.c64 = e64[0].p;
+    a.t64 = ncols > 1 ? e64[1].p : nullptr;
+    a.c32 = e64Stale[0] ? e32[0].p : nullptr;
+    a.t32 = ncols > 1 && e64Stale[1] ? e32[1].p : nullptr;
+    a.tconst = ncols > 1 ? 0.0 : 100000.0 / 2;
+    J.branchOf = wBranch.p;
+    J.tconst = a.tconst;
+    for (int k = 0; k < 2; ++k) {
+        J.recNodes[k] = bRecNodes[k].p;
+        J.recEdges[k] = bRecEdges[k].p;
+        J.recC[k] = bRecC[k].p;
+        J.recT[k] = bRecT[k].p;
+    }
+    J.cap = cap;
+    J.status = PAIR_PENDING;
+    Control c{};
+    c.epoch = ctlEpoch;
+    PGC_CUDA(cudaMemcpyAsync(wCtl.p, &c, sizeof(Control), cudaMemcpyHostToDevice, stream));
+}
+
 void Graph::batch_begin(int K, PairJob& J, int threads, int ctas, size_t smemCap, bool regenerate) {
     const auto t0 = std::chrono::steady_clock::now();
     if (regenerate) generate();
@@ -1627,58 +1734,27 @@ void Graph::batch_begin(int K, PairJob& J, int threads, int ctas, size_t smemCap
     batchThreads = 0;
     batchSmem = r.smemBytes;
     reset_predecessors();
-    // PGC_BATCH_CYCLE_CAP (tests): a smaller record, so that graphs are
-    // handed back to the host
-    const long long capMax = std::min<long long>(kBatchCycleCap, std::max(1, env_int("PGC_BATCH_CYCLE_CAP", (int)kBatchCycleCap)));
-    const int cap = (int)std::min<long long>(numNodes() + 4, capMax);
-    for (int k = 0; k < 2; ++k) {
-        bRecNodes[k].alloc((size_t)cap + 1);
-        bRecEdges[k].alloc((size_t)cap);
-        bRecC[k].alloc((size_t)cap);
-        bRecT[k].alloc((size_t)cap);
-    }
-    J = PairJob{};
-    J.bf = params(r, 0, 0, 0.0, std::numeric_limits<float>::infinity());
-    J.bf.ctaSlice = wCtaSlice.p;
-    J.ctas = r.blocks;
-    J.threads = r.threads;
-    LookupArgs& a = J.lk;
-    a.n = T.n;
-    a.nY = T.nY;
-    a.nodeSlot = dNodeSlot.p;
-    a.numNodes = numNodes();
-    a.eBlock = T.eBlock;
-    a.spInter = dSp[INTER].p;
-    a.spIntra = dSp[INTRA].p;
-    a.srcInter = dSrc[INTER].p;
-    a.srcDummy = dSrcDummy.p ? dSrcDummy.p : dSrc[INTER].p;
-    a.srcIntra = dSrc[INTRA].p;
-    a.tedgeInter = dTedge[INTER].p;
-    a.tedgeIntra = dTedge[INTRA].p;
-    a.interEntries = T.entries[INTER];
-    a.layerStride = T.layerStride();
-    a.c64 = e64[0].p;
-    a.t64 = ncols > 1 ? e64[1].p : nullptr;
-    a.c32 = e64Stale[0] ? e32[0].p : nullptr;
-    a.t32 = ncols > 1 && e64Stale[1] ? e32[1].p : nullptr;
-    a.tconst = ncols > 1 ? 0.0 : scaling / 2;
-    J.branchOf = wBranch.p;
-    J.tconst = a.tconst;
-    for (int k = 0; k < 2; ++k) {
-        J.recNodes[k] = bRecNodes[k].p;
-        J.recEdges[k] = bRecEdges[k].p;
-        J.recC[k] = bRecC[k].p;
-        J.recT[k] = bRecT[k].p;
-    }
-    J.cap = cap;
-    J.status = PAIR_PENDING;
-    Control c{};
-    c.epoch = ctlEpoch;
-    PGC_CUDA(cudaMemcpyAsync(wCtl.p, &c, sizeof(Control), cudaMemcpyHostToDevice, stream));
+    fill_job(r, J);
     PGC_CUDA(sync_stream());
 }
 
 void Graph::batch_end(const PairJob& J) {
+    stats.launches += 1;
+    const long long launches = stats.launches;
+    finish_job(J, batchK);
+    if (J.status != PAIR_HOST) {
+        stats.launches += launches;
+        DeviceInfo info{};
+        if (device_info(device, &info) == cudaSuccess && info.clockKhz > 0)
+            stats.deviceMs += (double)J.cycles / info.clockKhz;  // the team's time on this graph at the top SM clock
+    }
+}
+
+// The result from a finished job, or the solve finished on the host when the
+// device handed it back; statistics of the solve but for its launches and its
+// device time.
+void Graph::finish_job(const PairJob& J, int K) {
+    stats = Stats();
     Control c{};
     d2h(&c, wCtl.p, sizeof(Control));
     PGC_CUDA(sync_stream());
@@ -1689,7 +1765,6 @@ void Graph::batch_end(const PairJob& J) {
     stats.candidates = J.candidates;
     stats.fallbackWalks = J.fallbackWalks;
     stats.branches = 1;
-    stats.launches += 1;
     // the lead thread's cycle counters, summed over the solve's calls
     stats.cycA = c.cycPhaseA;
     stats.cycB = c.cycPhaseB;
@@ -1699,14 +1774,10 @@ void Graph::batch_end(const PairJob& J) {
     stats.cycCand = c.cycCand;
     stats.cycLead = c.cycLead;
     stats.cycStage = c.cycStage;
-    stats.steps = J.sweeps * ((long long)(T.nY + 1) * (T.entries[INTRA] == 0 ? 1 : batchK) - 1);
-    {
-        DeviceInfo info{};
-        if (device_info(device, &info) == cudaSuccess && info.clockKhz > 0)
-            stats.deviceMs = (double)J.cycles / info.clockKhz;  // the CTA's time on this graph at the top SM clock
-    }
+    stats.steps = J.sweeps * ((long long)(T.nY + 1) * (T.entries[INTRA] == 0 ? 1 : K) - 1);
     stats.ctas = J.ctas;
     stats.threads = J.threads;
+    stats.waitEntries = J.ctas > 1 ? waitEntries : 0;
     switch (J.status) {
         case PAIR_DONE: {
             std::vector<long long> edges((size_t)std::max(0, J.nEdges));
@@ -1732,8 +1803,23 @@ void Graph::batch_end(const PairJob& J) {
             // branch and bound (or a cycle longer than the device record):
             // the host's solve from the rescaled costs
             stats = Stats();
-            solve_ratio_rescaled(batchK);
+            solve_ratio_rescaled(K);
             return;
+        case PAIR_WRAPS: {
+            FirstBranch first{J.bound, J.lambda, {}};
+            const size_t m = (size_t)J.nEdges;
+            first.cycle.nodes.resize(m + 1);
+            first.cycle.edges.resize(m);
+            first.cycle.c.resize(m);
+            first.cycle.t.resize(m);
+            d2h(first.cycle.nodes.data(), bRecNodes[J.rec].p, sizeof(int) * (m + 1));
+            d2h(first.cycle.edges.data(), bRecEdges[J.rec].p, sizeof(long long) * m);
+            d2h(first.cycle.c.data(), bRecC[J.rec].p, sizeof(double) * m);
+            d2h(first.cycle.t.data(), bRecT[J.rec].p, sizeof(double) * m);
+            PGC_CUDA(sync_stream());
+            solve_ratio_rescaled(K, &first);
+            return;
+        }
         case PAIR_ERR_WAIT:
             wLayerFlag.zero(stream);
             ctlEpoch = 0;
@@ -2558,13 +2644,13 @@ int pgc_solve_batch(pgc_graph* const* graphs, int64_t count, const char* solver,
             // device.  The costs are generated and rescaled per graph by the
             // workers first; graphs whose first branch's cycle wraps are
             // finished on the host afterwards, with branch and bound.
-            const size_t smemCap = (size_t)std::max(0, info.smemOptin / pgc::kBatchBlocksPerSm - 2560);
-            // Relaxing threads per CTA: 20 warps, or 8 for graphs whose mean
-            // fits 8 slices.  CTAs per team (ctas_per_graph, else
-            // PGC_BATCH_TEAM, else a mean share of one slice per warp, as a
-            // power of two of at most 16): a team relaxes a graph's steps side
-            // by side, so more CTAs per graph shorten each solve; fewer solve
-            // more graphs at once.
+            const size_t smemCap = (size_t)std::max(0, info.smemOptin - pgc::kBatchStaticSmem);
+            // Threads per CTA: 20 warps, or 8 for graphs whose mean fits 8
+            // slices (a warp of them stages).  CTAs per team (ctas_per_graph,
+            // else PGC_BATCH_TEAM, else a mean share of one slice per warp, as
+            // a power of two of at most 16): a team relaxes a graph's steps
+            // side by side, so more CTAs per graph shorten each solve; fewer
+            // solve more graphs at once.
             double slices = 0;
             int64_t live = 0;
             for (int64_t i = 0; i < count; ++i) {
@@ -2578,7 +2664,7 @@ int pgc_solve_batch(pgc_graph* const* graphs, int64_t count, const char* solver,
             int team = ctas_per_graph > 0 ? ctas_per_graph : pgc::env_int("PGC_BATCH_TEAM", 0);
             if (team <= 0)
                 for (team = 1; team < 16 && team * (threads / 32) < slices;) team *= 2;
-            team = std::max(1, std::min(team, sms * pgc::kBatchBlocksPerSm));
+            team = std::max(1, std::min(team, sms));
             const unsigned spin = (unsigned)std::max(1, pgc::env_int("PGC_BF_SPIN_LIMIT", (int)pgc::kDefaultSpinLimit));
             std::vector<PairJob> jobs((size_t)count);
             std::vector<int> costF32((size_t)count, 0), timeKind((size_t)count, 0);
@@ -2651,7 +2737,7 @@ int pgc_solve_batch(pgc_graph* const* graphs, int64_t count, const char* solver,
                     while (k1 < order.size() && costF32[(size_t)order[k1]] == cf && timeKind[(size_t)order[k1]] == tk)
                         smem = std::max(smem, smemNeed[(size_t)order[k1++]]);
                     int perSm = 0;
-                    PGC_CUDA(pgc::bf_batch_max_blocks(cf, tk, threads + 32, smem, &perSm));
+                    PGC_CUDA(pgc::bf_batch_max_blocks(cf, tk, threads, smem, &perSm));
                     if (perSm < 1) throw Failure(PGC_ERR_CUDA, "the batched solve kernel cannot be resident");
                     // whole teams, all resident (the launch is cooperative
                     // when a team has more than one CTA)
@@ -2663,7 +2749,7 @@ int pgc_solve_batch(pgc_graph* const* graphs, int64_t count, const char* solver,
                     g_batchProfile[6] = threads;
                     g_batchProfile[7] = std::max(g_batchProfile[7], (double)smem);
                     PGC_CUDA(pgc::launch_bf_batch(dJobs.p + k0, (int)(k1 - k0), dNext.p + grp % 8, dTeamWords.p, g,
-                                                  spin, cf, tk, blocks, threads + 32, smem, bs));
+                                                  spin, cf, tk, blocks, threads, smem, bs));
                     k0 = k1;
                 }
                 PGC_CUDA(cudaMemcpyAsync(packed.data(), dJobs.p, sizeof(PairJob) * packed.size(),
@@ -2674,7 +2760,7 @@ int pgc_solve_batch(pgc_graph* const* graphs, int64_t count, const char* solver,
             g_batchProfile[1] = ms_since(tKernel);
             const auto tEnd = std::chrono::steady_clock::now();
             for (const PairJob& J : jobs) {
-                if (J.status == pgc::PAIR_HOST) g_batchProfile[3] += 1;
+                if (J.status == pgc::PAIR_HOST || J.status == pgc::PAIR_WRAPS) g_batchProfile[3] += 1;
                 if (J.status == pgc::PAIR_DONE || J.status == pgc::PAIR_NAN) g_batchProfile[4] += 1;
             }
             for_each_graph([&](int64_t i) {
