@@ -404,6 +404,12 @@ cudaError_t launch_lookup_pairs(const LookupArgs& a, cudaStream_t stream);
 // column's pass takes a grid proportional to its entries
 cudaError_t launch_plain_energy(const EnergyArgs& a, cudaStream_t s, bool shared = false);
 cudaError_t launch_ho_energy(const EnergyArgs& a, cudaStream_t s);
+struct FdMax {
+    double value;
+    long long at;
+};
+constexpr int kFdMaxBlocks = 592;  // four blocks per SM
+cudaError_t launch_fd_max(const double* fd, long long n, FdMax* part, cudaStream_t s);
 cudaError_t launch_quaternions(const QuatArgs& a, cudaStream_t s);
 // Median of a column and its rescale (cost_time_ratio_solver.cpp:709-721),
 // enqueued whole on stream s (kernels_energy.cu).

@@ -422,6 +422,7 @@ class Graph {
     double adjLambda = 0;     // the ratio result's C / T in double
     double fdMax = 0;         // maxFd of the ("*", "feature") time column, as the energy used it
     long long fdArgmax = 0;   // the first feat_diff entry holding the maximum
+    DBuf<FdMax> wFdMax;
     DBuf<long long> wAdjEdges;
     DBuf<double> wImport;
     // `wait`: finish the stream before returning (batched callers wait once
@@ -431,8 +432,7 @@ class Graph {
     void set_feat_diff(const double* fd, int64_t rows, int64_t cols);
     void set_feat_diff_device(const double* fd, int64_t rows, int64_t cols, bool wait = true);
     // After set_feat_diff_device the matrix lives only in dFD; the host copy
-    // is read back when a host reader needs it (the feature-time maximum, the
-    // CSV export).
+    // is read back when a host reader needs it (the CSV export).
     bool fdHostStale = false;
     void ensure_fd_host();
 
@@ -644,17 +644,14 @@ void Graph::generate() {
         a.rlPwr = rlPwr;
         a.maxSO3 = (double)(float)robust_loss_host(2 * M_PI, rlAlpha, rlC, rlPwr);
         if (tm == FEATURE) {
-            ensure_fd_host();
-            double m = -std::numeric_limits<double>::infinity();
-            long long at = 0;
-            for (size_t i = 0; i < FD.size(); ++i)
-                if (FD[i] > m) {
-                    m = FD[i];
-                    at = (long long)i;
-                }
-            a.maxFd = (double)(float)m;
+            wFdMax.alloc(kFdMaxBlocks + 1);
+            PGC_CUDA(launch_fd_max(dFD.p, (long long)(nvx * nvy), wFdMax.p, s));
+            FdMax top{};
+            d2h(&top, wFdMax.p + kFdMaxBlocks, sizeof(FdMax));
+            PGC_CUDA(sync_stream());
+            a.maxFd = (double)(float)top.value;
             fdMax = a.maxFd;
-            fdArgmax = at;
+            fdArgmax = top.at;
         }
         if (reg) {
             dNX.upload(NX.data(), NX.size(), s);
