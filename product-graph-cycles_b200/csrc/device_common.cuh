@@ -191,12 +191,18 @@ struct QuatArgs {
     double4* out;
 };
 
+// A column's streams: (nY + 1) layers of layerStride entries, the interlayer
+// rows first; per row of 32 entries of a layer, the lanes that hold an edge.
+struct StreamView {
+    long long layerStride, interEntries;
+    int nY;
+    const unsigned* rowMask;  // [layerStride / 32]
+};
+
 struct SelectArgs {
     const double* col;
-    long long total, layerStride, interEntries;
-    int nY;
-    const int* tedgeInter;
-    const int* tedgeIntra;
+    long long total;
+    StreamView view;
     unsigned long long* hist;  // 1 << kMedianWideBits counters
 };
 
@@ -420,10 +426,9 @@ cudaError_t launch_median_rescale(const SelectArgs& a, unsigned long long* topHi
                                   double scaling, float* col32, double clip, bool allPasses, bool shared,
                                   cudaStream_t s);
 cudaError_t launch_rescale_f64(const SelectArgs& a, MedianState* st, double clip, cudaStream_t s);
-cudaError_t launch_to_f64(const float* col32, double* col, long long layerStride, long long interEntries, int nY,
-                          const int* ti, const int* tr, cudaStream_t s);
-cudaError_t launch_to_f32(const double* col, float* col32, long long total, long long layerStride,
-                          long long interEntries, int nY, const int* ti, const int* tr, int* exact, cudaStream_t s);
+cudaError_t launch_to_f64(const float* col32, double* col, const StreamView& view, cudaStream_t s);
+cudaError_t launch_to_f32(const double* col, float* col32, const StreamView& view, int* exact, cudaStream_t s);
+cudaError_t launch_row_masks(const int* tedge, long long entries, unsigned* mask, cudaStream_t s);
 cudaError_t launch_export(const double* col, double* out, int cols, int c, long long total, long long layerStride,
                           long long interEntries, int nY, long long eBlock, const int* ti, const int* tr,
                           cudaStream_t s);

@@ -38,93 +38,55 @@ __device__ __forceinline__ double line_integral(const EnergyArgs& a, int y0, int
     return sqrt(li);
 }
 
-// Visits the per-layer streams in work items of consecutive positions of one
-// layer (one division per item, not per entry): f(idx, l, pos, t, inRange)
-// for every position; t is the template edge, >= 0 for a real edge (l >= 1
-// for interlayer entries, l < nY for intralayer ones).  Positions are visited
-// warp-aligned, so every lane of a warp makes the same calls (warp
-// collectives inside f are allowed); lanes past the item's end get
-// inRange = false.
-template <class F>
-__device__ __forceinline__ void for_stream_layers(long long layerStride, long long interEntries, int nY,
-                                                  const int* ti, const int* tr, F f) {
-    // Two positions per thread and round: their template ids are loaded
-    // together, and f reads its tables through the read-only path (__ldg), so
-    // the compiler may overlap the two positions' table reads with the
-    // other's stores.  Positions inside a layer fit 32 bits.
-    constexpr int U = 2;
-    const int stride = (int)layerStride, inter = (int)interEntries;
-    const int chunk = 8 * (int)blockDim.x;  // a multiple of U * blockDim.x
-    const int perLayer = (stride + chunk - 1) / chunk;
-    const long long items = (long long)perLayer * (nY + 1);
-    const int lane = threadIdx.x & 31, step = (int)blockDim.x;
-    for (long long it = blockIdx.x; it < items; it += gridDim.x) {
-        const int l = (int)(it / perLayer);
-        const int p0 = (int)(it - (long long)l * perLayer) * chunk;
-        const int p1 = min(p0 + chunk, stride);
-        const long long rowBase = (long long)l * layerStride;
-        const int* tInter = l >= 1 ? ti : nullptr;
-        const int* tIntra = l < nY ? tr - inter : nullptr;
-        for (int base = p0 + (int)threadIdx.x; base - lane < p1; base += U * step) {
-            int t[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int pos = base + u * step;
-                const int* tb = pos < inter ? tInter : tIntra;
-                t[u] = (pos < p1 && tb) ? __ldg(tb + pos) : -1;
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int pos = base + u * step;
-                if (pos - lane < p1) f(rowBase + pos, l, (long long)pos, t[u], pos < p1);
-            }
-        }
-    }
-}
-
-// The same visit for passes that read one column: f(idx, x, valid, inRange)
-// with x = col[idx] (0 where !inRange).  Each thread first loads U positions
-// (template ids and values) and then calls f on them, so U loads of each
-// stream are in flight per thread however much f synchronises; one load at
-// a time left a pass at about a quarter of HBM bandwidth.
+// Visits a column's streams two neighbouring positions at a time: f(idx, x, m)
+// for every pair, idx the even position's index, bit u of m set where entry
+// idx + u holds an edge.  Which list slots hold one is the same in every layer
+// and known per row of 32 (StreamView::rowMask; layer 0 has no interlayer
+// edges, layer nY no intralayer ones), so a pass reads 16 bytes of column per
+// lane and one mask word per row instead of a template id per entry; each
+// thread has U such loads in flight.  Work items are chunks of one layer, one
+// division each.
 template <int U, class F>
-__device__ __forceinline__ void for_stream_values(const double* col, long long layerStride, long long interEntries,
-                                                  int nY, const int* ti, const int* tr, F f) {
-    // positions inside a layer fit 32 bits (the streams of one layer are
-    // indexed by int slot offsets), which keeps the U-fold unrolled body small
-    const int stride = (int)layerStride, inter = (int)interEntries;
-    const int chunk = 8 * (int)blockDim.x;  // a multiple of U * blockDim.x
-    const int perLayer = (stride + chunk - 1) / chunk;
-    const long long items = (long long)perLayer * (nY + 1);
-    const int lane = threadIdx.x & 31, step = (int)blockDim.x;
-    for (long long it = blockIdx.x; it < items; it += gridDim.x) {
+__device__ __forceinline__ void for_stream_pairs(const double* col, const StreamView& v, F f) {
+    const int stride = (int)v.layerStride, inter = (int)v.interEntries;  // positions inside a layer fit 32 bits
+    const int step = 2 * (int)blockDim.x, chunk = 2 * U * step;
+    const unsigned perLayer = (unsigned)((stride + chunk - 1) / chunk);
+    const unsigned items = perLayer * (unsigned)(v.nY + 1);
+    for (unsigned it = blockIdx.x; it < items; it += gridDim.x) {
         const int l = (int)(it / perLayer);
-        const int p0 = (int)(it - (long long)l * perLayer) * chunk;
-        const int p1 = min(p0 + chunk, stride);
-        const long long rowBase = (long long)l * layerStride;
+        const int p0 = (int)(it - (unsigned)l * perLayer) * chunk + 2 * (int)threadIdx.x;
+        const int p1 = min(p0 - 2 * (int)threadIdx.x + chunk, stride);
+        const long long rowBase = (long long)l * v.layerStride;
         const double* row = col + rowBase;
-        const int* tInter = l >= 1 ? ti : nullptr;
-        const int* tIntra = l < nY ? tr - inter : nullptr;
-        for (int base = p0 + (int)threadIdx.x; base - lane < p1; base += U * step) {
-            int t[U];
-            double x[U];
+        const int lo = l == 0 ? inter : 0, hi = l == v.nY ? inter : stride;  // positions that can hold an edge
+        for (int base = p0; base < p1; base += U * step) {
+            double2 x[U];
+            unsigned m[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const int pos = base + u * step;
-                t[u] = -1;
-                x[u] = 0.0;
+                m[u] = 0;
+                x[u] = make_double2(0.0, 0.0);
                 if (pos < p1) {
-                    const int* tb = pos < inter ? tInter : tIntra;
-                    if (tb) t[u] = tb[pos];
-                    x[u] = row[pos];
+                    x[u] = *reinterpret_cast<const double2*>(row + pos);
+                    if (pos >= lo && pos < hi) m[u] = (__ldg(v.rowMask + (pos >> 5)) >> (pos & 31)) & 3u;
                 }
             }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const int pos = base + u * step;
-                if (pos - lane < p1) f(rowBase + pos, x[u], t[u] >= 0, pos < p1);
+                if (pos < p1) f(rowBase + pos, x[u], m[u]);
             }
         }
+    }
+}
+
+// Which lanes of every list row hold an edge.
+__global__ void row_mask_kernel(const int* tedge, long long entries, unsigned* mask) {
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < entries;
+         e += (long long)gridDim.x * blockDim.x) {  // whole warps: entries is a multiple of 32
+        const unsigned m = __ballot_sync(0xffffffffu, tedge[e] >= 0);
+        if ((threadIdx.x & 31) == 0) mask[e >> 5] = m;
     }
 }
 
@@ -757,20 +719,22 @@ __global__ void median_hist_kernel(SelectArgs a, const MedianState* st) {
     // warp matching) would serialise.
     unsigned runBin = 0xffffffffu, runCnt = 0;
     const unsigned long long prefix = m.prefix, mask = m.mask;
-    for_stream_values<4>(a.col, a.layerStride, a.interEntries, a.nY, a.tedgeInter, a.tedgeIntra,
-                         [&](long long, double x, bool valid, bool) {
-                             if (!valid) return;
-                             const unsigned long long k = order_key(x);
-                             if ((k & mask) != prefix) return;
-                             const unsigned bin = (unsigned)((k >> shift) & (unsigned long long)(nb - 1));
-                             if (bin == runBin) {
-                                 ++runCnt;
-                             } else {
-                                 if (runCnt) atomicAdd(&sh[runBin], runCnt);
-                                 runBin = bin;
-                                 runCnt = 1;
-                             }
-                         });
+    auto take = [&](double x) {
+        const unsigned long long k = order_key(x);
+        if ((k & mask) != prefix) return;
+        const unsigned bin = (unsigned)((k >> shift) & (unsigned long long)(nb - 1));
+        if (bin == runBin) {
+            ++runCnt;
+        } else {
+            if (runCnt) atomicAdd(&sh[runBin], runCnt);
+            runBin = bin;
+            runCnt = 1;
+        }
+    };
+    for_stream_pairs<4>(a.col, a.view, [&](long long, double2 x, unsigned m) {
+        if (m & 1u) take(x.x);
+        if (m & 2u) take(x.y);
+    });
     if (runCnt) atomicAdd(&sh[runBin], runCnt);
     __syncthreads();
     for (int i = threadIdx.x; i < nb; i += blockDim.x)
@@ -780,7 +744,8 @@ __global__ void median_hist_kernel(SelectArgs a, const MedianState* st) {
 // Block-wide search of a histogram of nb bins (1024 threads): the digit whose
 // cumulative count first exceeds `rank`, and the count below it.  Returns
 // false when the counts do not reach past the rank.
-__device__ bool find_digit(const unsigned long long* hist, int nb, long long rank, int* digit, long long* below) {
+template <class Count>
+__device__ bool find_digit(const Count* hist, int nb, long long rank, int* digit, long long* below) {
     __shared__ long long part[1024];
     __shared__ int sDigit;
     __shared__ long long sBelow;
@@ -873,12 +838,15 @@ __global__ void median_compact_kernel(SelectArgs a, MedianState* st, double* out
     }
     if (m.shift == 0 || m.err) return;
     const unsigned long long prefix = m.prefix, mask = m.mask;
-    for_stream_values<4>(a.col, a.layerStride, a.interEntries, a.nY, a.tedgeInter, a.tedgeIntra,
-                         [&](long long, double x, bool valid, bool) {
-                           if (!valid || (order_key(x) & mask) != prefix) return;
-                           const unsigned long long at = atomicAdd(count, 1ull);
-                           if ((long long)at < cap) out[at] = x;
-                       });
+    auto take = [&](double x) {
+        if ((order_key(x) & mask) != prefix) return;
+        const unsigned long long at = atomicAdd(count, 1ull);
+        if ((long long)at < cap) out[at] = x;
+    };
+    for_stream_pairs<4>(a.col, a.view, [&](long long, double2 x, unsigned m) {
+        if (m & 1u) take(x.x);
+        if (m & 2u) take(x.y);
+    });
 }
 
 // The order statistics inside the last bucket (one block of 1024 threads):
@@ -888,7 +856,7 @@ __global__ void median_compact_kernel(SelectArgs a, MedianState* st, double* out
 // Radix selection over the bucket's remaining bits, 11 at a time.
 __global__ void median_select_kernel(MedianState* st, const double* band, const unsigned long long* count) {
     __shared__ MedianState m;
-    __shared__ unsigned long long hist[1 << 11];
+    __shared__ unsigned hist[1 << 11];  // a bucket holds at most kMedianCompact values
     __shared__ unsigned long long sMin;
     __shared__ long long sLess, sEq;
     if (threadIdx.x == 0) m = *st;
@@ -928,7 +896,7 @@ __global__ void median_select_kernel(MedianState* st, const double* band, const 
                 for (int u = 0; u < 8; ++u) {
                     if (i0 + (long long)u * blockDim.x >= n) break;
                     const unsigned long long k = order_key(x[u]);
-                    if ((k & mask) == prefix) atomicAdd(&hist[(k >> shift) & (unsigned long long)(nb - 1)], 1ull);
+                    if ((k & mask) == prefix) atomicAdd(&hist[(k >> shift) & (unsigned long long)(nb - 1)], 1u);
                 }
             }
             __syncthreads();
@@ -1006,12 +974,14 @@ __global__ void median_min_above_kernel(SelectArgs a, MedianState* st) {
     if (!m.needAbove || m.err) return;
     const unsigned long long above = m.bucketTop;
     unsigned long long best = ~0ull;
-    for_stream_values<4>(a.col, a.layerStride, a.interEntries, a.nY, a.tedgeInter, a.tedgeIntra,
-                         [&](long long, double x, bool valid, bool) {
-                           if (!valid) return;
-                           const unsigned long long k = order_key(x);
-                           if (k > above && k < best) best = k;
-                       });
+    auto take = [&](double x) {
+        const unsigned long long k = order_key(x);
+        if (k > above && k < best) best = k;
+    };
+    for_stream_pairs<4>(a.col, a.view, [&](long long, double2 x, unsigned m) {
+        if (m & 1u) take(x.x);
+        if (m & 2u) take(x.y);
+    });
     for (int o = 16; o > 0; o >>= 1) {
         const unsigned long long x = __shfl_xor_sync(0xffffffffu, best, o);
         best = x < best ? x : best;
@@ -1037,9 +1007,8 @@ __device__ __forceinline__ double median_factor(const MedianState& m, double sca
 // The factor comes from the selection (the first pass, writeF64 == 0, also
 // stores it and the median in the state) or, for the second pass, from the
 // state; nothing is written when the selection failed.
-__global__ void rescale_kernel(double* col, float* col32, long long layerStride, long long interEntries, int nY,
-                               const int* tedgeInter, const int* tedgeIntra, MedianState* st, double scaling,
-                               double clip, int writeF64) {
+__global__ void rescale_kernel(double* col, float* col32, StreamView view, MedianState* st, double scaling, double clip,
+                               int writeF64) {
     __shared__ double sFactor;
     __shared__ int sErr;
     if (threadIdx.x == 0) {
@@ -1057,46 +1026,56 @@ __global__ void rescale_kernel(double* col, float* col32, long long layerStride,
     __syncthreads();
     if (sErr) return;
     const double factor = sFactor;
-    int* inexact = &st->inexact;
-    for_stream_values<4>(col, layerStride, interEntries, nY, tedgeInter, tedgeIntra,
-                         [&](long long idx, double v, bool valid, bool inRange) {
-                           if (!inRange) return;
-                           if (!valid) {
-                               if (col32) col32[idx] = __int_as_float(0x7fc00000);
-                               return;
-                           }
-                           double x = round(__dmul_rn(factor, v));
-                           if (x > clip) x = clip;
-                           if (writeF64) col[idx] = x;
-                           const float f = (float)x;
-                           if (col32) col32[idx] = f;
-                           if ((double)f != x) *inexact = 1;
-                       });
+    const float nan = __int_as_float(0x7fc00000);
+    bool inexact = false;
+    auto scaled = [&](double v) {
+        const double x = round(__dmul_rn(factor, v));
+        return x > clip ? clip : x;
+    };
+    for_stream_pairs<4>(col, view, [&](long long idx, double2 v, unsigned m) {
+        float2 f = make_float2(nan, nan);
+        if (m & 1u) {
+            const double x = scaled(v.x);
+            f.x = (float)x;
+            inexact |= (double)f.x != x;
+            if (writeF64) col[idx] = x;
+        }
+        if (m & 2u) {
+            const double x = scaled(v.y);
+            f.y = (float)x;
+            inexact |= (double)f.y != x;
+            if (writeF64) col[idx + 1] = x;
+        }
+        if (col32) *reinterpret_cast<float2*>(col32 + idx) = f;
+    });
+    if (inexact) st->inexact = 1;
 }
 // The double column from its exact float copy, on the valid entries.
-__global__ void to_f64_kernel(const float* col32, double* col, long long layerStride, long long interEntries, int nY,
-                              const int* tedgeInter, const int* tedgeIntra) {
-    for_stream_layers(layerStride, interEntries, nY, tedgeInter, tedgeIntra,
-                      [&](long long idx, int, long long, int t, bool inRange) {
-                          if (inRange && t >= 0) col[idx] = (double)col32[idx];
-                      });
+__global__ void to_f64_kernel(const float* col32, double* col, StreamView view) {
+    // the visit's loads of the double column are not used, and not made
+    for_stream_pairs<4>(col, view, [&](long long idx, double2, unsigned m) {
+        const float2 f = *reinterpret_cast<const float2*>(col32 + idx);
+        if (m & 1u) col[idx] = (double)f.x;
+        if (m & 2u) col[idx + 1] = (double)f.y;
+    });
 }
 
-__global__ void to_f32_kernel(const double* col, float* col32, long long total, long long layerStride,
-                              long long interEntries, int nY, const int* tedgeInter, const int* tedgeIntra,
-                              int* exact) {
-    (void)total;
-    for_stream_values<4>(col, layerStride, interEntries, nY, tedgeInter, tedgeIntra,
-                         [&](long long idx, double x, bool valid, bool inRange) {
-                           if (!inRange) return;
-                           if (!valid) {
-                               col32[idx] = __int_as_float(0x7fc00000);
-                               return;
-                           }
-                           const float f = (float)x;
-                           col32[idx] = f;
-                           if ((double)f != x) *exact = 0;
-                       });
+__global__ void to_f32_kernel(const double* col, float* col32, StreamView view, int* exact) {
+    const float nan = __int_as_float(0x7fc00000);
+    bool inexact = false;
+    for_stream_pairs<4>(col, view, [&](long long idx, double2 x, unsigned m) {
+        float2 f = make_float2(nan, nan);
+        if (m & 1u) {
+            f.x = (float)x.x;
+            inexact |= (double)f.x != x.x;
+        }
+        if (m & 2u) {
+            f.y = (float)x.y;
+            inexact |= (double)f.y != x.y;
+        }
+        *reinterpret_cast<float2*>(col32 + idx) = f;
+    });
+    if (inexact) *exact = 0;
 }
 
 __global__ void export_kernel(const double* col, double* out, int cols, int c, long long total,
@@ -1590,8 +1569,7 @@ cudaError_t launch_median_rescale(const SelectArgs& a, unsigned long long* topHi
     note_launch();
     median_min_above_kernel<<<grid, 256, 0, s>>>(a, st);
     note_launch();
-    rescale_kernel<<<grid, 256, 0, s>>>(const_cast<double*>(a.col), col32, a.layerStride, a.interEntries, a.nY,
-                                        a.tedgeInter, a.tedgeIntra, st, scaling, clip, 0);
+    rescale_kernel<<<grid, 256, 0, s>>>(const_cast<double*>(a.col), col32, a.view, st, scaling, clip, 0);
     return cudaGetLastError();
 }
 
@@ -1599,22 +1577,24 @@ cudaError_t launch_median_rescale(const SelectArgs& a, unsigned long long* topHi
 // float copy is not exact).
 cudaError_t launch_rescale_f64(const SelectArgs& a, MedianState* st, double clip, cudaStream_t s) {
     note_launch();
-    rescale_kernel<<<stream_grid(rescale_kernel, 256, 0), 256, 0, s>>>(const_cast<double*>(a.col), nullptr,
-                                                                        a.layerStride, a.interEntries, a.nY,
-                                                                        a.tedgeInter, a.tedgeIntra, st, 0.0, clip, 1);
+    rescale_kernel<<<stream_grid(rescale_kernel, 256, 0), 256, 0, s>>>(const_cast<double*>(a.col), nullptr, a.view, st,
+                                                                        0.0, clip, 1);
     return cudaGetLastError();
 }
-cudaError_t launch_to_f64(const float* col32, double* col, long long layerStride, long long interEntries, int nY,
-                          const int* ti, const int* tr, cudaStream_t s) {
+cudaError_t launch_to_f64(const float* col32, double* col, const StreamView& view, cudaStream_t s) {
     note_launch();
-    to_f64_kernel<<<stream_grid(to_f64_kernel, 256, 0), 256, 0, s>>>(col32, col, layerStride, interEntries, nY, ti, tr);
+    to_f64_kernel<<<stream_grid(to_f64_kernel, 256, 0), 256, 0, s>>>(col32, col, view);
     return cudaGetLastError();
 }
-cudaError_t launch_to_f32(const double* col, float* col32, long long total, long long layerStride,
-                          long long interEntries, int nY, const int* ti, const int* tr, int* exact, cudaStream_t s) {
+cudaError_t launch_to_f32(const double* col, float* col32, const StreamView& view, int* exact, cudaStream_t s) {
     note_launch();
-    to_f32_kernel<<<stream_grid(to_f32_kernel, 256, 0), 256, 0, s>>>(col, col32, total, layerStride, interEntries, nY, ti, tr,
-                                                       exact);
+    to_f32_kernel<<<stream_grid(to_f32_kernel, 256, 0), 256, 0, s>>>(col, col32, view, exact);
+    return cudaGetLastError();
+}
+cudaError_t launch_row_masks(const int* tedge, long long entries, unsigned* mask, cudaStream_t s) {
+    if (entries == 0) return cudaSuccess;
+    note_launch();
+    row_mask_kernel<<<grid_for(entries, 256), 256, 0, s>>>(tedge, entries, mask);
     return cudaGetLastError();
 }
 cudaError_t launch_export(const double* col, double* out, int cols, int c, long long total, long long layerStride,

@@ -316,6 +316,7 @@ class Graph {
     int ncols = 1;
     DBuf<int> dSlotNode, dNodeSlot, dSp[2], dSrc[2], dTedge[2], dSrcDummy, dEX, dEY, dESrc, dETrgt, dEXcols;
     DBuf<int8_t> dEYpat, dENext;
+    DBuf<unsigned> dRowMask;
     DBuf<double> dVX, dVY, dFD, dNX, dNY;
     DBuf<double4> dQuat;
     DBuf<double> e64[2];
@@ -411,6 +412,9 @@ class Graph {
     DBuf<unsigned long long> topHist[2];
     bool topHistValid[2] = {false, false};
     EnergyArgs energy_args() const;
+    StreamView stream_view() const {
+        return StreamView{T.layerStride(), T.entries[INTER], T.nY, dRowMask.p};
+    }
 
     // What the adjoint of the last solve needs: the product of the rescale
     // factors applied to each cost column since its costs were last set, the
@@ -544,6 +548,9 @@ void Graph::upload_template() {
         dSrc[p].upload(T.src[p].data(), T.src[p].size(), s);
         dTedge[p].upload(T.tedge[p].data(), T.tedge[p].size(), s);
     }
+    dRowMask.alloc((size_t)T.layerStride() / 32);
+    for (int p = 0; p < 2; ++p)
+        PGC_CUDA(launch_row_masks(dTedge[p].p, T.entries[p], dRowMask.p + (p ? T.entries[INTER] / 32 : 0), s));
     dSlotNode.upload(T.slotNode.data(), T.slotNode.size(), s);
     dNodeSlot.upload(T.nodeSlot.data(), T.nodeSlot.size(), s);
     // The closing layer's source list differs from the interlayer one only
@@ -714,11 +721,7 @@ void Graph::rescale_columns(double scaling) {
         SelectArgs a{};
         a.col = e64[col].p;
         a.total = total;
-        a.layerStride = stride;
-        a.interEntries = T.entries[INTER];
-        a.nY = T.nY;
-        a.tedgeInter = dTedge[INTER].p;
-        a.tedgeIntra = dTedge[INTRA].p;
+        a.view = stream_view();
         return a;
     };
     auto enqueue = [&](int col, bool allPasses) {
@@ -769,8 +772,7 @@ void Graph::rescale_columns(double scaling) {
 
 void Graph::ensure_e64(int col) {
     if (!e64Stale[col]) return;
-    PGC_CUDA(launch_to_f64(e32[col].p, e64[col].p, T.layerStride(), T.entries[INTER], T.nY, dTedge[INTER].p,
-                           dTedge[INTRA].p, stream));
+    PGC_CUDA(launch_to_f64(e32[col].p, e64[col].p, stream_view(), stream));
     stats.launches++;
     e64Stale[col] = false;
 }
@@ -784,8 +786,7 @@ void Graph::ensure_f32(int col) {
     wCount.alloc(1);
     const int one = 1;
     PGC_CUDA(cudaMemcpyAsync(wCount.p, &one, sizeof(int), cudaMemcpyHostToDevice, stream));
-    PGC_CUDA(launch_to_f32(e64[col].p, e32[col].p, total, stride, T.entries[INTER], T.nY, dTedge[INTER].p,
-                           dTedge[INTRA].p, wCount.p, stream));
+    PGC_CUDA(launch_to_f32(e64[col].p, e32[col].p, stream_view(), wCount.p, stream));
     stats.launches++;
     int exact = 0;
     d2h(&exact, wCount.p, sizeof(int));
