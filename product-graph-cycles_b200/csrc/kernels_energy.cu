@@ -132,78 +132,98 @@ __device__ __forceinline__ void top_digit_end(const EnergyArgs& a, unsigned* sh,
     }
 }
 
-// Each thread takes U = 4 positions of one layer per round and walks them
-// through the entry's chain of dependent reads one level at a time --
-// template edge id, then its Y pattern and X columns, then the two feat_diff
-// entries -- so each level's U loads are in flight together (one position
-// at a time left the kernel at a tenth of HBM bandwidth on small graphs).
-// The arithmetic per entry is deformationEnergy.cpp:11-78's, unchanged.
-__global__ void plain_energy_kernel(EnergyArgs a) {
+// Work item: a block of template positions x a chunk of layers.  A thread
+// keeps its position -- template edge, Y pattern, X columns, the X half of the
+// line integral -- and walks the chunk's layers four at a time, so that per
+// entry it reads only two feat_diff entries, neighbours in their rows of the
+// ones it read a layer before, and a warp's stores stay 32 consecutive entries
+// of one layer.  (Walking every entry through template edge, columns and
+// feat_diff again took 235 us a graph of the 64-pair batch, 47 us for 2.6
+// million entries of one graph.)  The arithmetic per entry is
+// deformationEnergy.cpp:11-78's, in its order.
+__global__ void __launch_bounds__(256) plain_energy_kernel(EnergyArgs a, int layerChunk) {
     extern __shared__ unsigned int topSh[];  // [2][kTopBins] when a.hist0
     const double nan = __longlong_as_double(0x7ff8000000000000LL);
     DigitRun r0, r1;
     top_digit_begin(a, topSh);
     constexpr int U = 4;
-    const int stride = (int)a.layerStride, inter = (int)a.interEntries;
-    const int chunk = U * (int)blockDim.x;
-    const int perLayer = (stride + chunk - 1) / chunk;
-    const long long items = (long long)perLayer * (a.nY + 1);
-    const int step = (int)blockDim.x;
+    const int stride = (int)a.layerStride, inter = (int)a.interEntries, layers = a.nY + 1;
+    const int posBlocks = (stride + (int)blockDim.x - 1) / (int)blockDim.x;
+    const int chunks = (layers + layerChunk - 1) / layerChunk;
+    const long long items = (long long)posBlocks * chunks;
     for (long long it = blockIdx.x; it < items; it += gridDim.x) {
-        const int l = (int)(it / perLayer);
-        const int p0 = (int)(it - (long long)l * perLayer) * chunk;
-        const long long rowBase = (long long)l * a.layerStride;
-        const int* tInter = l >= 1 ? a.tedgeInter : nullptr;
-        const int* tIntra = l < a.nY ? a.tedgeIntra - inter : nullptr;
-        const int yInter0 = l >= 1 ? __ldg(a.EY + 2 * (l - 1)) : 0, yInter1 = l >= 1 ? __ldg(a.EY + 2 * (l - 1) + 1) : 0;
-        const int yIntra0 = l < a.nY ? __ldg(a.EY + 2 * l) : 0, yIntra1 = l < a.nY ? __ldg(a.EY + 2 * l + 1) : 0;
-        int t[U], y0[U], y1[U], x0[U], x1[U];
-        double f0[U], f1[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int pos = p0 + u * step + (int)threadIdx.x;
-            const int* tb = pos < inter ? tInter : tIntra;
-            t[u] = (pos < stride && tb) ? __ldg(tb + pos) : -2;  // -2: out of range, -1: empty slot
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int pos = p0 + u * step + (int)threadIdx.x;
-            y0[u] = y1[u] = x0[u] = x1[u] = 0;
-            if (t[u] >= 0) {
-                const bool interPos = pos < inter;
-                y0[u] = interPos ? yInter0 : yIntra0;
-                y1[u] = __ldg(a.eY + t[u]) == 0 ? y0[u] : (interPos ? yInter1 : yIntra1);
-                x0[u] = __ldg(a.eX + 3 * t[u]);
-                x1[u] = __ldg(a.eX + 3 * t[u] + 1);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            f0[u] = f1[u] = 0.0;
-            if (t[u] >= 0) {
-                f0[u] = __ldg(a.FD + (long long)x0[u] * a.nvy + y0[u]);
-                f1[u] = __ldg(a.FD + (long long)x1[u] * a.nvy + y1[u]);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int pos = p0 + u * step + (int)threadIdx.x;
-            if (t[u] == -2 && pos < stride) t[u] = -1;  // a slot of a layer side without edges
-            if (pos >= stride) continue;
-            const long long idx = rowBase + pos;
-            if (t[u] < 0) {
+        const int lc = (int)(it / posBlocks);
+        const int pos = (int)(it - (long long)lc * posBlocks) * (int)blockDim.x + (int)threadIdx.x;
+        if (pos >= stride) continue;
+        const int l0 = lc * layerChunk, l1 = min(l0 + layerChunk, layers);
+        const bool isInter = pos < inter;
+        const int t = isInter ? __ldg(a.tedgeInter + pos) : __ldg(a.tedgeIntra + (pos - inter));
+        if (t < 0) {
+            for (int l = l0; l < l1; ++l) {
+                const long long idx = (long long)l * stride + pos;
                 a.out0[idx] = nan;
                 if (a.out1) a.out1[idx] = nan;
-                continue;
             }
-            const double li = a.lineIntegral ? line_integral(a, y0[u], y1[u], x0[u], x1[u]) : 1.0;
-            const double fd = f0[u] + f1[u];
-            const double c0 = a.lengthMode ? fd : 0.5 * fd * li;
-            a.out0[idx] = c0;
-            if (a.lengthMode) a.out1[idx] = li;
-            if (a.hist0) {
-                count_top_digit(topSh, r0, c0);
-                if (a.hist1) count_top_digit(topSh + kTopBins, r1, li);
+            continue;
+        }
+        const bool ahead = __ldg(a.eY + t) != 0;  // the second vertex is the next one of Y
+        const int x0 = __ldg(a.eX + 3 * t), x1 = __ldg(a.eX + 3 * t + 1);
+        const double* fd0 = a.FD + (long long)x0 * a.nvy;
+        const double* fd1 = a.FD + (long long)x1 * a.nvy;
+        double dxx[3] = {0.0, 0.0, 0.0};
+        if (a.lineIntegral) {
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                const double dx = __ldg(a.VX + 3 * x0 + j) - __ldg(a.VX + 3 * x1 + j);
+                dxx[j] = dx * dx;
+            }
+        }
+        for (int lu = l0; lu < l1; lu += U) {
+            int y0[U], y1[U];
+            double f0[U], f1[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int b = isInter ? lu + u - 1 : lu + u;
+                y0[u] = -1;
+                if (lu + u < l1 && b >= 0 && b < a.nY) {
+                    y0[u] = __ldg(a.EY + 2 * b);
+                    y1[u] = ahead ? __ldg(a.EY + 2 * b + 1) : y0[u];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (y0[u] >= 0) {
+                    f0[u] = __ldg(fd0 + y0[u]);
+                    f1[u] = __ldg(fd1 + y1[u]);
+                }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (lu + u >= l1) break;
+                const long long idx = (long long)(lu + u) * stride + pos;
+                if (y0[u] < 0) {  // no edge in this layer's slot
+                    a.out0[idx] = nan;
+                    if (a.out1) a.out1[idx] = nan;
+                    continue;
+                }
+                double li = 1.0;
+                if (a.lineIntegral) {  // line_integral's sum, in its order
+                    li = 0.0;
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) {
+                        const double dy = __ldg(a.VY + 3 * y0[u] + j) - __ldg(a.VY + 3 * y1[u] + j);
+                        li = li + dy * dy;
+                        li = li + dxx[j];
+                    }
+                    li = sqrt(li);
+                }
+                const double fd = f0[u] + f1[u];
+                const double c0 = a.lengthMode ? fd : 0.5 * fd * li;
+                a.out0[idx] = c0;
+                if (a.lengthMode) a.out1[idx] = li;
+                if (a.hist0) {
+                    count_top_digit(topSh, r0, c0);
+                    if (a.hist1) count_top_digit(topSh + kTopBins, r1, li);
+                }
             }
         }
     }
@@ -1490,7 +1510,10 @@ static int grid_for(long long total, int threads) {
 cudaError_t launch_plain_energy(const EnergyArgs& a, cudaStream_t s, bool shared) {
     const size_t smem = a.hist0 ? 2 * kTopBins * sizeof(unsigned) : 0;
     note_launch();
-    plain_energy_kernel<<<stream_grid(plain_energy_kernel, 256, smem, shared ? a.total : -1), 256, smem, s>>>(a);
+    // sixteen layers a thread, fewer where that would leave SMs idle: a wave of
+    // four blocks per SM takes chunks of four layers up to 2.4 M entries
+    const int chunk = a.total < 148LL * 4 * 256 * 16 ? 4 : 16;
+    plain_energy_kernel<<<stream_grid(plain_energy_kernel, 256, smem, shared ? a.total : -1), 256, smem, s>>>(a, chunk);
     return cudaGetLastError();
 }
 cudaError_t launch_ho_energy(const EnergyArgs& a, cudaStream_t s) {
