@@ -889,14 +889,18 @@ Graph::Run Graph::prepare_run(int K, bool ratio) {
     if (envThreads && (envThreads < 32 || envThreads > kBfThreads || envThreads % 32 != 0))
         throw Failure(PGC_ERR_ARG, "PGC_BF_THREADS must be a multiple of 32 in [32, 640]");
     {
-        // Teams on local tables: one CTA while a step's relaxation is shorter
-        // than an exchange, else CTAs of a few slices each, up to one per SM.
+        // Teams on local tables: CTAs of six slices, up to one per SM, and one
+        // CTA for up to eight slices.  An exchange costs 1.3k cycles and a
+        // slice more on the same schedulers about 0.15k: 162 x 20 (6 slices)
+        // takes 0.56 ms with one CTA and 0.72 with two, 642 x 60 (21 slices)
+        // 1.08 with one and 2, 1.02 with four, 1.10 with eleven, 1,777 x 97 (56)
+        // 5.3 ms with CTAs of four slices, 4.5 of six, 4.6 of eight, 5.4 of 19.
         int active = 0;
         for (int s = 0; s < T.nslices; ++s)
             if (T.sp[INTER][(size_t)s + 1] > T.sp[INTER][(size_t)s]) ++active;
         int lb = envBlocks;
         if (lb <= 0) {
-            lb = active <= env_int("PGC_BF_LOCAL_ONE", 24) ? 1 : (active + env_int("PGC_BF_LOCAL_SL", 4) - 1) / env_int("PGC_BF_LOCAL_SL", 4);
+            lb = active <= 8 ? 1 : (active + 5) / 6;
             if (teamCap > 0) lb = std::min(lb, teamCap);
         }
         lb = std::max(1, std::min({lb, T.nslices, sms}));
@@ -2649,19 +2653,23 @@ int pgc_solve_batch(pgc_graph* const* graphs, int64_t count, const char* solver,
             // a power of two of at most 16): a team relaxes a graph's steps
             // side by side, so more CTAs per graph shorten each solve; fewer
             // solve more graphs at once.
-            double slices = 0;
+            // A share of more than 32 slices of the largest graph would not fit
+            // a CTA's tables, and that graph would hold up the launch.
+            double slices = 0, most = 0;
             int64_t live = 0;
             for (int64_t i = 0; i < count; ++i) {
                 if (!graphs[i]) continue;
                 const Graph& g = graphs[i]->g;
-                slices += g.conj ? 3.0 * (double)g.nex / 32 : (double)g.nvx / 32;
+                const double own = g.conj ? 3.0 * (double)g.nex / 32 : (double)g.nvx / 32;
+                slices += own;
+                most = std::max(most, own);
                 ++live;
             }
             slices /= (double)std::max<int64_t>(1, live);
             const int threads = slices <= 8 ? 256 : pgc::kBatchThreads;
             int team = ctas_per_graph > 0 ? ctas_per_graph : pgc::env_int("PGC_BATCH_TEAM", 0);
             if (team <= 0)
-                for (team = 1; team < 16 && team * (threads / 32) < slices;) team *= 2;
+                for (team = 1; team < 16 && (team * (threads / 32) < slices || team * 32 < most);) team *= 2;
             team = std::max(1, std::min(team, sms));
             const unsigned spin = (unsigned)std::max(1, pgc::env_int("PGC_BF_SPIN_LIMIT", (int)pgc::kDefaultSpinLimit));
             std::vector<PairJob> jobs((size_t)count);
