@@ -343,7 +343,7 @@ def measure_pair(args, world, rank, workload, steps, warmup, e2e_steps, with_min
         achieved = (b_sweep * t["sweeps"]) / (t["bf_us"] * 1e-6) / 1e9 if t["bf_us"] else None
         r = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
              "frac": (achieved / peak) if achieved else None, "traffic": None,
-             "peak_kind": f"{peak_kind} hbm_gbs", "kernel": "bf_kernel",
+             "peak_kind": f"{peak_kind} hbm_gbs", "kernel": "bf_batch_kernel" if ratio_mode else "bf_local_kernel",
              "algorithmic_bytes_per_sweep": b_sweep, "sweeps_per_solve": t["sweeps"] / steps_done,
              "bf_ms_per_solve": t["bf_us"] / 1000.0 / steps_done}
         if ratio_mode:

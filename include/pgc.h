@@ -180,7 +180,7 @@ int pgc_set_team_shape(pgc_graph* g, int ctas, int threads_per_cta);
  * Ratio solvers: `workers` host threads (0: 64) generate and rescale every
  * graph's costs; then one persistent launch runs each graph's whole ratio
  * solve on the device, teams of `ctas_per_graph` CTAs (0: the environment's
- * PGC_BATCH_TEAM, else 8) taking the graphs largest first; a graph whose
+ * PGC_BATCH_TEAM, else by the graphs' sizes) taking the graphs largest first; a graph whose
  * first-branch cycle wraps is finished on the host with branch and bound.
  * PGC_BATCH_STREAMS=1 selects the route of the other solvers instead.
  * Other solvers: each graph on its own stream with a team of at most

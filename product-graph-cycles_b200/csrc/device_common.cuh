@@ -122,7 +122,7 @@ struct BfParams {
     int* candStat;                 // [n] shortcut verdict per candidate (0 none, 1 cycle, 2 no cycle, 3 undecided)
     int* candV0;                   // [n] first repeated layer-0 node of a candidate's walk
     long long* candSteps;          // [n] predecessor steps that walk needs
-    int* layerFlag;                // [nY+1] stamp of the last sweep that improved the layer
+    int* layerFlag;                // [nY+1] stamp of the last sweep that improved the layer (local tables: layer nY - 1 only)
     const int* branchOf;
     int branchId;
     double lambda, ub;
@@ -249,7 +249,7 @@ struct LookupArgs {
     double* tOut;
 };
 
-// One graph of a batched ratio solve (bf_batch_kernel): a CTA takes the job
+// One graph of a ratio solve on the device (bf_batch_kernel): a team takes the job
 // from the queue and runs its whole solve on the device -- the initial upper
 // bound (cost_time_ratio_solver.cpp:652-707), the Lawler iterations
 // (:558-635) and their cycle evaluations (computeRatioForCycle, :88-133) --

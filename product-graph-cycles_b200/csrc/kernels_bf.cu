@@ -1583,14 +1583,14 @@ __global__ void lookup_pairs_kernel(LookupArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// Batched ratio solves.  Each CTA takes graphs from a queue and runs the
-// host driver's ratio solve on the device for each: the initial upper bound
-// (cost_time_ratio_solver.cpp:652-707), the Lawler iterations (:558-635)
-// with their Bellman-Ford calls as one-CTA teams, and the cycle evaluations
-// (computeRatioForCycle, :88-133) in the same double operations and order as
-// the host.  The first branch's Lawler result is the solve's result unless
-// its cycle wraps (:840-850); then the host takes the graph over with branch
-// and bound, and the device's work on it only cost time.
+// Ratio solves, of one graph or of many.  Teams of CTAs take graphs from a
+// queue and run the host driver's ratio solve on the device for each: the
+// initial upper bound (cost_time_ratio_solver.cpp:652-707), the Lawler
+// iterations (:558-635) with their Bellman-Ford calls, and the cycle
+// evaluations (computeRatioForCycle, :88-133) in the same double operations
+// and order as the host.  The first branch's Lawler result is the solve's
+// result unless its cycle wraps (:840-850); then the host goes on from that
+// cycle with branch and bound.
 // ---------------------------------------------------------------------------
 namespace {
 

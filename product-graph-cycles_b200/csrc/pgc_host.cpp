@@ -448,7 +448,7 @@ class Graph {
     // device's solve in `job`; then the result taken from the finished job, or the
     // solve finished on the host when the device handed it back.
     void batch_begin(int K, PairJob& job, int threads, int ctas, size_t smemCap, bool regenerate);
-    void batch_end(const PairJob& job);
+    void batch_end(const PairJob& job, int ctas);
     int batchK = 0;
     size_t batchSmem = 0;  // dynamic shared memory the prepared batch team needs
     size_t batch_smem_bytes() const { return batchSmem; }
@@ -1740,9 +1740,15 @@ void Graph::batch_begin(int K, PairJob& J, int threads, int ctas, size_t smemCap
     PGC_CUDA(sync_stream());
 }
 
-void Graph::batch_end(const PairJob& J) {
+void Graph::batch_end(const PairJob& J, int ctas) {
     stats.launches += 1;
     const long long launches = stats.launches;
+    struct Cap {  // a graph handed back keeps to the caller's team size
+        int& cap;
+        const int saved;
+        ~Cap() { cap = saved; }
+    } restore{teamCap, teamCap};
+    if (ctas > 0) teamCap = ctas;
     finish_job(J, batchK);
     if (J.status != PAIR_HOST) {
         stats.launches += launches;
@@ -2774,7 +2780,7 @@ int pgc_solve_batch(pgc_graph* const* graphs, int64_t count, const char* solver,
                     Graph& g = graphs[i]->g;
                     g.blockingSync = true;
                     try {
-                        g.batch_end(jobs[(size_t)i]);
+                        g.batch_end(jobs[(size_t)i], ctas_per_graph);
                     } catch (...) {
                         g.blockingSync = false;
                         throw;

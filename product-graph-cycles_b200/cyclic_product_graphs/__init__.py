@@ -453,7 +453,7 @@ def solve_batch(generators, solver_name: str, max_depth: int | None = None, ctas
     Ratio solvers: ``workers`` native threads (0: 64) generate and rescale the
     costs, then one persistent launch runs every graph's whole ratio solve on
     the device, teams of ``ctas_per_graph`` CTAs (0: ``PGC_BATCH_TEAM``, else
-    8) taking the graphs largest first; a graph whose first-branch cycle wraps
+    by the graphs' sizes) taking the graphs largest first; a graph whose first-branch cycle wraps
     is finished on the host with branch and bound.  Other solvers run each
     graph on its own CUDA stream with a team of at most ``ctas_per_graph``
     CTAs (0: SMs / min(graphs, 32)); the device runs those streams side by
