@@ -22,11 +22,11 @@
 // acquire hand-off of per-CTA step counters with two CTA barriers around it
 // (still there for more than four depths and for tables that do not fit).
 // Cycles per step, before -> now (relaxation + hand-off or exchange):
-//   conjugate 5,000 x 200, K = 3, 148 CTAs     6.0k + 3.8k -> 2.3k + 2.3k
-//   pruned 20,000 x 500, 148 CTAs             25.7k + 5.4k -> 11.3k + 4.1k
-//   plain 1,777 x 97, K = 3, 3 -> 14 CTAs      5.9k + 2.7k -> 1.7k + 1.8k
-//   plain 642 x 60, K = 2, one CTA             5.5k + 0.5k -> 3.8k + 0.2k
-//   64 uneven plain pairs in one launch       11.7k + 4.6k -> 2-4k + 1.5k
+//   conjugate 5,000 x 200, K = 3, 148 CTAs     6.0k + 3.8k -> 2.1k + 2.2k
+//   pruned 20,000 x 500, 148 CTAs             25.7k + 5.4k -> 9.3k + 2.9k
+//   plain 1,777 x 97, K = 3, 3 -> 10 CTAs      5.9k + 2.7k -> 1.8k + 1.3k
+//   plain 642 x 60, K = 2, 1 -> 4 CTAs         5.5k + 0.5k -> 1.5k + 1.3k
+//   64 uneven plain pairs in one launch       11.7k + 4.6k -> 2.7k + 1.5k
 // What bounds it now: shared-memory wavefronts of the source reads and issue
 // slots where an SM holds a slice per warp, the dependent chain of one slice
 // where it holds few, and the L2 round trip of the exchange.
