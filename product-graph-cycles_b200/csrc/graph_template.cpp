@@ -236,13 +236,22 @@ void build_conj(const int* EX, int64_t nEX, LayerTemplate& T) {
 // a contiguous range of slices holds all kinds of its edges.
 void mesh_order(const int* EX, int64_t nEX, LayerTemplate& T) {
     const int nv = T.conj ? T.nvx : T.n;
-    std::vector<int> ptr((size_t)nv + 1, 0), out((size_t)nEX), order;
-    for (int64_t e = 0; e < nEX; ++e) ++ptr[(size_t)EX[2 * e] + 1];
+    // Out-edges of every vertex in ascending edge order.  Edges that come
+    // sorted by their source, as mesh tools write them, are that list already
+    // (`out` stays empty).
+    std::vector<int> ptr((size_t)nv + 1, 0), out, order;
+    bool sorted = true;
+    for (int64_t e = 0; e < nEX; ++e) {
+        ++ptr[(size_t)EX[2 * e] + 1];
+        sorted &= e == 0 || EX[2 * e] >= EX[2 * e - 2];
+    }
     for (int v = 0; v < nv; ++v) ptr[(size_t)v + 1] += ptr[(size_t)v];
-    {
+    if (!sorted) {
+        out.resize((size_t)nEX);
         std::vector<int> fill(ptr.begin(), ptr.end() - 1);
         for (int64_t e = 0; e < nEX; ++e) out[(size_t)fill[(size_t)EX[2 * e]]++] = (int)e;
     }
+    auto edge = [&](int q) { return sorted ? q : out[(size_t)q]; };
     order.reserve((size_t)nv);
     std::vector<unsigned char> seen((size_t)nv, 0);
     for (int r = 0; r < nv; ++r) {
@@ -253,7 +262,7 @@ void mesh_order(const int* EX, int64_t nEX, LayerTemplate& T) {
         for (; head < order.size(); ++head) {
             const int v = order[head];
             for (int q = ptr[(size_t)v]; q < ptr[(size_t)v + 1]; ++q) {
-                const int w = EX[2 * out[(size_t)q] + 1];
+                const int w = EX[2 * edge(q) + 1];
                 if (seen[(size_t)w]) continue;
                 seen[(size_t)w] = 1;
                 order.push_back(w);
@@ -279,7 +288,7 @@ void mesh_order(const int* EX, int64_t nEX, LayerTemplate& T) {
         for (int q = ptr[(size_t)v]; q < ptr[(size_t)v + 1]; ++q, ++rank)
             for (int kind = 0; kind < 3; ++kind) {
                 const int slot = (int)(((rank >> 5) * 3 + kind) * 32 + (rank & 31));
-                const int node = kind * (int)nEX + out[(size_t)q];
+                const int node = kind * (int)nEX + edge(q);
                 T.slotNode[(size_t)slot] = node;
                 T.nodeSlot[(size_t)node] = slot;
             }
