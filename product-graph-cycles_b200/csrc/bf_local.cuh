@@ -414,7 +414,7 @@ __device__ __forceinline__ void local_stage_issue(int b, int l, int k) {
     if (TK) bulk_load(dst + (size_t)H.rowCap * 32 * costBytes, H.time + base * timeBytes, bt, H.bar + b);
 }
 
-// Once per launch: the CTA's tables and its in-edges' local source indices.
+// At the start of a call: the CTA's tables and its in-edges' local source indices.
 __device__ __forceinline__ void local_begin(const BfParams& p, const Team& t, int s0, int s1, int costBytes,
                                             int timeBytes) {
     LocalHot& H = local_hot();

@@ -249,6 +249,12 @@ __device__ __forceinline__ unsigned smem_addr(const void* p) {
 __device__ __forceinline__ void mbar_init(unsigned long long* bar) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar)) : "memory");
 }
+// The word is an mbarrier no longer: it may hold other data, or be
+// initialised again.  A launch makes many Bellman-Ford calls, and PTX leaves
+// an init of a live mbarrier, or a plain store over one, undefined.
+__device__ __forceinline__ void mbar_inval(unsigned long long* bar) {
+    asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
 __device__ __forceinline__ void mbar_expect(unsigned long long* bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes)
                  : "memory");
@@ -890,7 +896,7 @@ __device__ int dij_walk_end(const BfParams& p, int v) {
 // all of the dynamic shared memory; the number keeps the kernels' instances of
 // the step loop apart.
 template <class CT, int TK, bool S, int SITE = 0>
-__device__ __forceinline__ void bf_body(const BfParams& p, const Team& t, char* smem) {
+__device__ __forceinline__ void bf_run(const BfParams& p, const Team& t, char* smem, unsigned long long* stageBar) {
     constexpr bool LOCAL = SITE > 0;
     const int n = p.n, K = p.K, Kp = p.Kp;
     const long long tid = t.thread(), nth = t.nthreads();
@@ -900,7 +906,6 @@ __device__ __forceinline__ void bf_body(const BfParams& p, const Team& t, char* 
     if (handoff && threadIdx.x == 0) p.stepDone[(size_t)t.cta * kStepDoneStride] = 0;
     // shared memory: [row offsets of both parts][slices with rows, per part]
     // [step buffer 0][step buffer 1]
-    __shared__ unsigned long long stageBar[2];
     __shared__ int nActive[2];
     Stage st;
     if constexpr (!LOCAL) {
@@ -1391,6 +1396,28 @@ __device__ __forceinline__ void bf_body(const BfParams& p, const Team& t, char* 
         if (isLead) atomicAdd(&p.ctl->cycTail, clock64() - tTail);
         if (!tailOk || finished) return;
     }
+}
+
+// bf_run between the two mbarriers' first and last use: it initialises them
+// (with the CTA's lists or tables) and leaves them at one point of the code for
+// the whole CTA; they are given up here, so that the next call of the launch
+// finds plain memory.
+template <class CT, int TK, bool S, int SITE = 0>
+__device__ __forceinline__ void bf_body(const BfParams& p, const Team& t, char* smem) {
+    unsigned long long* bar;
+    if constexpr (SITE > 0) {
+        bar = local_hot().bar;
+    } else {
+        __shared__ unsigned long long stageBar[2];
+        bar = stageBar;
+    }
+    bf_run<CT, TK, S, SITE>(p, t, smem, bar);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        mbar_inval(bar);
+        mbar_inval(bar + 1);
+    }
+    __syncthreads();
 }
 
 // The Bellman-Ford launch of one graph.  Every CTA of the grid belongs to

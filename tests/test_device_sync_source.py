@@ -1,0 +1,39 @@
+"""Rules of the device code's synchronisation that no run shows: a GPU does what
+one expects when they are broken, until it does not.  Read from the sources."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "product-graph-cycles_b200", "csrc")
+
+
+@pytest.fixture(scope="module")
+def functions():
+    """Body of every function of the Bellman-Ford sources, comments removed."""
+    out = {}
+    for name in ("kernels_bf.cu", "bf_local.cuh"):
+        with open(os.path.join(CSRC, name)) as f:
+            text = re.sub(r"//[^\n]*", "", f.read())
+        for m in re.finditer(r"^(?!\s|#|template|struct|namespace|using|constexpr|static_assert|extern)[^;={}]*?(\w+)\([^{};]*\)\s*\{\n",
+                             text, re.M):
+            end = text.index("\n}", m.end() - 1)
+            out[m.group(1)] = text[m.end():end]
+    return out
+
+
+def _callers(functions, name):
+    return {f for f, body in functions.items() if re.search(r"\b%s\s*[<(]" % name, body)}
+
+
+def test_an_mbarrier_ends_before_its_words_are_used_again(functions):
+    """Every mbarrier.init belongs to a Bellman-Ford call that invalidates both
+    words after its last use (a launch makes many calls)."""
+    assert {f for f, body in functions.items() if "mbarrier.init." in body} == {"mbar_init"}
+    assert _callers(functions, "mbar_init") == {"bf_run", "local_begin"}
+    assert _callers(functions, "local_begin") == {"bf_run"}
+    assert _callers(functions, "bf_run") == {"bf_body"}
+    body = functions["bf_body"]
+    after = body[body.index("bf_run<"):]
+    assert re.search(r"__syncthreads\(\);.*mbar_inval\(bar\);.*mbar_inval\(bar \+ 1\);.*__syncthreads\(\);", after, re.S)
+    assert "mbarrier.inval.shared::cta.b64" in functions["mbar_inval"]
