@@ -589,11 +589,15 @@ __device__ bool relax_step(const BfParams& p, const Stage& st, int sb, int s0, i
 // CTA is complete; publish it, then wait until every CTA on this CTA's wait
 // list (the owners of the sources it reads and the readers of the rows it
 // overwrites next) has completed it too.  This replaces a grid-wide barrier:
-// a CTA waits only for its graph neighbours.  Returns false when a wait ran
-// out of iterations or another CTA raised the error word.  The CTA named by
+// a CTA waits only for its graph neighbours.  Returns false, to every thread
+// of the CTA or to none, when a wait ran out of iterations or another CTA
+// raised the error word: one thread reads that word for the CTA (another CTA
+// may raise it between two threads' reads, and the CTA's next barriers need
+// all of it).  The CTA named by
 // p.stallCta (a test hook; -1 in every solve) also waits for a word that no
 // code writes, so its wait runs out.
 __device__ bool step_handoff(const BfParams& p, const Team& t, unsigned step) {
+    __shared__ int sGood;
     __syncthreads();  // the CTA's writes of this step are done
     if (threadIdx.x < 32) {
         // release store: with the CTA barrier above it publishes every write
@@ -612,7 +616,7 @@ __device__ bool step_handoff(const BfParams& p, const Team& t, unsigned step) {
                 const bool ready = f == nullptr || (int)(ld_acquire_u32(f) - step) >= 0;
                 if (__all_sync(0xffffffffu, ready)) break;
                 ++spins;
-                if ((spins & 63u) == 0 && *(volatile int*)t.err) { good = 0; break; }
+                if (__any_sync(0xffffffffu, (spins & 63u) == 0 && *(volatile int*)t.err)) { good = 0; break; }
                 if (spins > t.spin) {
                     if (threadIdx.x == 0) atomicExch(t.err, 1);
                     good = 0;
@@ -621,10 +625,13 @@ __device__ bool step_handoff(const BfParams& p, const Team& t, unsigned step) {
                 if (spins > 256) __nanosleep(32);
             }
         }
-        if (threadIdx.x == 0 && !good) atomicExch(t.err, 1);
+        if (threadIdx.x == 0) {
+            if (!good) atomicExch(t.err, 1);
+            sGood = good && *(volatile int*)t.err == 0;
+        }
     }
     __syncthreads();
-    return *(volatile int*)t.err == 0;
+    return sGood != 0;
 }
 
 #include "bf_local.cuh"

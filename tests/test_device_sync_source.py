@@ -37,3 +37,14 @@ def test_an_mbarrier_ends_before_its_words_are_used_again(functions):
     after = body[body.index("bf_run<"):]
     assert re.search(r"__syncthreads\(\);.*mbar_inval\(bar\);.*mbar_inval\(bar \+ 1\);.*__syncthreads\(\);", after, re.S)
     assert "mbarrier.inval.shared::cta.b64" in functions["mbar_inval"]
+
+
+def test_a_cta_leaves_a_step_as_one(functions):
+    """The error word of a team is written by other CTAs at any time: the
+    threads of a CTA that read it one by one may disagree, and part of them
+    would miss the next barrier."""
+    body = functions["step_handoff"]
+    assert re.search(r"return sGood != 0;\s*$", body)
+    assert re.search(r"if \(threadIdx\.x == 0\) \{[^{}]*sGood = [^;]*t\.err[^;]*;\s*\}", body)
+    assert "__any_sync(0xffffffffu, (spins & 63u) == 0 && *(volatile int*)t.err)" in body
+    assert body.count("t.err") == body.count("atomicExch(t.err, 1)") + 2
