@@ -97,15 +97,18 @@ struct LocalHot {
     double lam, lt, ub;         // lambda, lambda times the constant time, upper bound
     long long layerStride, interEntries;
     unsigned long long cyc[3];  // lead: relaxation, exchange, waits for staged streams
-    // A wait of this CTA ran out in a step of that number modulo 4.  Set during
-    // the step, read by every warp between its barrier and the next one, and
-    // acted on before that one; later steps have words of their own, so every
-    // warp leaves at the same barrier.
+    // A wait of this CTA ran out in a step of that number modulo 4 (before the
+    // first step: in the one before it).  Set during the step, read by every
+    // warp between its barrier and the next one, and acted on before that one;
+    // later steps have words of their own, so every warp leaves at the same
+    // barrier.
     volatile int stop[4];
     int n, K, nY, nslots, L, nOwn, nHalo, s0, nsl, rowCap, hopBits;
     int r0[2], nrows[2], nAct[2];
     int nWait, stall, cta, ncta;
     unsigned spin;
+    unsigned copySpin;          // polls of the step loop's waits for copies (0: the test hook's CTA)
+    unsigned copiesOut;         // bit b: a copy into buffer b may be in flight after the sweep gave up
     unsigned oTslot, oGid, oHslot, oOh, oVal, oLsrc[2], oRec[2], oBuf[2];  // byte offsets in shared memory
 };
 static_assert(sizeof(LocalHot) <= kLocalHotBytes, "");
@@ -491,6 +494,8 @@ __device__ __forceinline__ void local_begin(const BfParams& p, const Team& t, in
             H.cta = t.cta;
             H.ncta = t.ncta;
             H.spin = p.spinLimit;
+            H.copySpin = t.cta == p.stallCopyCta ? 0u : p.spinLimit;
+            H.copiesOut = 0;
             H.oTslot = (unsigned)o.tslot;
             H.oGid = (unsigned)o.gid;
             H.oHslot = (unsigned)o.hslot;
@@ -589,7 +594,8 @@ __device__ __forceinline__ void local_store(const BfParams& p) {
 // stages the streams and waits for the neighbours' progress; the others relax
 // and take the halo; one CTA barrier ends each step.  `phase`: bit b is the
 // parity of step buffer b's next completion (kept by the last warp).  Returns
-// the new phases, bit 2 set when a wait ran out (no copy is in flight then).  SITE keeps the
+// the new phases, bit 2 set when a wait ran out; the copies are waited for once
+// more then, and H.copiesOut says whether that ran out too.  SITE keeps the
 // instances of kernels with different register budgets apart.
 template <class CT, int TK, int KD, int SITE>
 __device__ __noinline__ unsigned local_sweep(int stamp, unsigned step, unsigned phase) {
@@ -605,22 +611,33 @@ __device__ __noinline__ unsigned local_sweep(int stamp, unsigned step, unsigned 
         // barrier that opens their step: the relaxing warps read the buffer
         // without a wait of their own.
         const int lane = threadIdx.x & 31;
-        int stopped = 0;
+        unsigned out = 0;  // bit b: a copy into buffer b is in flight
         auto stage = [&](int b, int l, int k) {
             if (lane == 0) local_stage_issue<CT, TK>(b, l, k);
-            return ((staging >> (k == 0 ? 0 : 1)) & 1u) != 0;
+            const unsigned copy = (staging >> (k == 0 ? 0 : 1)) & 1u;
+            out |= copy << b;
+            return copy != 0;
+        };
+        auto wait = [&](int b, unsigned spin) {
+            if (!__all_sync(0xffffffffu, mbar_wait(H.bar + b, (phase >> b) & 1u, spin))) return false;
+            phase ^= 1u << b;
+            out &= ~(1u << b);
+            return true;
         };
         auto landed = [&](int b) {
-            if (!mbar_wait(H.bar + b, (phase >> b) & 1u, H.spin)) {
-                atomicExch(H.err, 1);
-                H.stop[step & 3] = 1;
-            }
-            phase ^= 1u << b;
+            if (wait(b, H.copySpin)) return;
+            atomicExch(H.err, 1);
+            H.stop[step & 3] = 1;
         };
         if (stage(0, KD > 1 ? 0 : 1, KD > 1 ? 1 : 0)) landed(0);
         __syncthreads();
+        int stopped = H.stop[step & 3];
         for (int l = KD > 1 ? 0 : 1; l <= nY && ok; ++l) {
             for (int k = l == 0 ? 1 : 0; k < (l == nY ? 1 : KD); ++k) {  // the closing layer has no intralayer edges
+                if (stopped) {
+                    ok = false;
+                    break;
+                }
                 const unsigned t0 = (unsigned)clock();
                 ++step;
                 if (l < nY) {
@@ -642,17 +659,17 @@ __device__ __noinline__ unsigned local_sweep(int stamp, unsigned step, unsigned 
                     if (copy) landed(sb ^ 1);
                     if (lane == 0 && H.cta == 0) H.cyc[2] += (unsigned)clock() - t0;
                 }
-                if (stopped) {
-                    ok = false;
-                    break;
-                }
                 __syncthreads();
                 if (lane == 0 && H.ncta > 1) st_relaxed_u32(H.stepDone + (size_t)H.cta * kStepDoneStride, step);
                 sb ^= 1;
                 stopped = H.stop[step & 3];
             }
         }
-        return phase | (ok && !stopped ? 0u : 4u);
+        if (ok && !stopped) return phase;
+        for (int b = 0; b < 2; ++b)
+            if ((out >> b) & 1u) wait(b, H.spin);
+        if (lane == 0) H.copiesOut = out;
+        return phase | 4u;
     }
     __syncthreads();  // the first step's streams have landed
     const bool lead = H.cta == 0 && threadIdx.x == 0;
@@ -671,7 +688,7 @@ __device__ __noinline__ unsigned local_sweep(int stamp, unsigned step, unsigned 
         }
     }
     const int predStep = (KD > 1 ? 1 : R.K) * R.n;
-    int stopped = 0;
+    int stopped = H.stop[step & 3];
     int predOff = predStep;
     for (int l = KD > 1 ? 0 : 1; l <= nY && ok; ++l) {
         for (int k = l == 0 ? 1 : 0; k < (l == nY ? 1 : KD); ++k) {

@@ -130,6 +130,7 @@ struct BfParams {
     int maxSweeps;                 // safety cap on sweeps in one launch (0 = unlimited)
     unsigned spinLimit;            // polls of any wait before it gives up and raises the error word
     int stallCta;                  // test hook (-1: none): this CTA's hand-off also waits on ctl->neverSet
+    int stallCopyCta;              // test hook (-1: none): this CTA's steps give their staged copies no poll
     int literalAll;                // test hook: decide every candidate by the literal walk
     Control* ctl;
     int* cycleBuf;                 // original node ids, walk order (reversed on the host)

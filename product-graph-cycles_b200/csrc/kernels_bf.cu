@@ -305,6 +305,7 @@ struct Stage {
     unsigned pending;            // bit b: copies issued into buffer b, not yet waited for
     int costBytes, timeBytes;    // bytes per entry of the cost and time streams
     unsigned spin;               // polls of a copy wait before it gives up
+    unsigned stepSpin;           // the same in the step loop (0: the test hook's CTA)
     __device__ const int* spl(int part) const { return part ? splIntra : splInter; }
     __device__ const int* act(int part) const { return part ? actIntra : actInter; }
     __device__ int nAct(int part) const { return part ? nActIntra : nActInter; }
@@ -348,19 +349,22 @@ __device__ void stage_issue(const BfParams& p, Stage& st, int s0, int s1, int b,
                   bt, st.bar + b);
 }
 
-// Wait for buffer b if copies were issued into it (every thread).
-__device__ __forceinline__ bool stage_wait(Stage& st, int b) {
+// Wait for buffer b if copies were issued into it (every thread).  A wait that
+// runs out leaves the copies pending.
+__device__ __forceinline__ bool stage_wait(Stage& st, int b, unsigned spin) {
     if (!((st.pending >> b) & 1u)) return true;
-    const bool ok = mbar_wait(st.bar + b, (st.phase >> b) & 1u, st.spin);
+    if (!mbar_wait(st.bar + b, (st.phase >> b) & 1u, spin)) return false;
     st.phase ^= 1u << b;
     st.pending &= ~(1u << b);
-    return ok;
+    return true;
 }
 
-// Before the CTA exits: no copy may still be writing its shared memory.
-__device__ __forceinline__ void stage_drain(Stage& st) {
-    stage_wait(st, 0);
-    stage_wait(st, 1);
+// Before the CTA leaves a call early: no copy may still be writing its shared
+// memory.  False, to every thread, when one may.
+__device__ __forceinline__ bool stage_drain(Stage& st) {
+    stage_wait(st, 0, st.spin);
+    stage_wait(st, 1, st.spin);
+    return __syncthreads_or((int)st.pending) == 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -903,7 +907,7 @@ __device__ int dij_walk_end(const BfParams& p, int v) {
 // all of the dynamic shared memory; the number keeps the kernels' instances of
 // the step loop apart.
 template <class CT, int TK, bool S, int SITE = 0>
-__device__ __forceinline__ void bf_run(const BfParams& p, const Team& t, char* smem, unsigned long long* stageBar) {
+__device__ __forceinline__ bool bf_run(const BfParams& p, const Team& t, char* smem, unsigned long long* stageBar) {
     constexpr bool LOCAL = SITE > 0;
     const int n = p.n, K = p.K, Kp = p.Kp;
     const long long tid = t.thread(), nth = t.nthreads();
@@ -951,6 +955,7 @@ __device__ __forceinline__ void bf_run(const BfParams& p, const Team& t, char* s
         st.rowCap = p.rowCap;
         st.srcOnly = p.stageSrcOnly != 0;
         st.spin = p.spinLimit;
+        st.stepSpin = t.cta == p.stallCopyCta ? 0u : p.spinLimit;
         const size_t bufBytes =
             bf_stage_buffer_bytes(p.rowCap, st.srcOnly ? 0 : st.costBytes, st.srcOnly ? 0 : st.timeBytes);
         st.buf0 = smem + bf_stage_offset(p.maxCtaSlices);
@@ -1004,7 +1009,7 @@ __device__ __forceinline__ void bf_run(const BfParams& p, const Team& t, char* s
         __syncthreads();
         if (threadIdx.x == 0) p.redAux[t.cta] = scnt;
     }
-    if (!team_sync(t)) return;
+    if (!team_sync(t)) return true;
     if (isLead) {
         int total = 0, last = -1;
         for (int c = 0; c < t.ncta; ++c) {
@@ -1017,11 +1022,11 @@ __device__ __forceinline__ void bf_run(const BfParams& p, const Team& t, char* s
         p.ctl->sweeps = 0;
         p.ctl->status = total == 0 ? BF_ERR_EMPTY_BRANCH : BF_RUNNING;
     }
-    if (!team_sync(t)) return;
-    if (*(volatile int*)&p.ctl->status != BF_RUNNING) return;
+    if (!team_sync(t)) return true;
+    if (*(volatile int*)&p.ctl->status != BF_RUNNING) return true;
 
     const int epochBase = p.ctl->epoch;  // read by all before anyone advances it
-    if (!team_sync(t)) return;
+    if (!team_sync(t)) return true;
     const int lastRow = p.nY % 2;
     const int lastPar = lastRow / K, lastDepth = lastRow % K;
     const long long numNodes = p.numNodes;
@@ -1040,8 +1045,8 @@ __device__ __forceinline__ void bf_run(const BfParams& p, const Team& t, char* s
         }
         for (long long i = tid; i < n; i += nth) p.bak[i] = ldV<S>(p, (size_t)i * Kp);
         if (!team_sync(t)) {
-            if constexpr (!LOCAL) stage_drain(st);
-            return;
+            if constexpr (LOCAL) return true;
+            else return stage_drain(st);
         }
         // Layers are relaxed in order; a CTA hands each step off to its
         // graph neighbours only (one team barrier closes the sweep).  The
@@ -1065,38 +1070,37 @@ __device__ __forceinline__ void bf_run(const BfParams& p, const Team& t, char* s
             }
             if (phase & 4u) {
                 atomicExch(t.err, 1);
-                return;
+                __syncthreads();
+                return H.copiesOut == 0;
             }
             step += (unsigned)(p.nY * p.localKD);
             local_store(p);
             cycRelax = H.cyc[0];
             cycHand = H.cyc[1];
             cycStage = H.cyc[2];
-            if (!team_sync(t)) return;
+            if (!team_sync(t)) return true;
         } else {
             int sb = 0;  // buffer of the current step
             for (int l = 0; l <= p.nY; ++l) {
                 for (int k = 0; k < kSteps; ++k) {
                     if (l == 0 && k == 0) continue;
                     const unsigned long long ta = isLead ? clock64() : 0;
-                    if (!stage_wait(st, sb)) {
-                        atomicExch(t.err, 1);
-                        stage_drain(st);
-                        return;
-                    }
+                    // a warp whose copies did not land raises the error word
+                    // and takes no part in the step
+                    const bool landed = __all_sync(0xffffffffu, stage_wait(st, sb, st.stepSpin));
+                    if (!landed) atomicExch(t.err, 1);
                     if (isLead) cycStage += clock64() - ta;
                     const bool last = l == p.nY && k == kSteps - 1;
                     if (!last) stage_issue(p, st, s0, s1, sb ^ 1, k + 1 < kSteps ? l : l + 1, k + 1 < kSteps ? k + 1 : 0);
-                    const bool any = relax_step<CT, TK, S>(p, st, sb, s0, s1, l, k);
+                    const bool any = landed && relax_step<CT, TK, S>(p, st, sb, s0, s1, l, k);
                     if (__any_sync(0xffffffffu, any) && (threadIdx.x & 31) == 0) p.layerFlag[l] = stamp;
                     const unsigned long long tb = isLead ? clock64() : 0;
                     ++step;
                     sb ^= 1;
-                    const bool ok = (handoff && !last) ? step_handoff(p, t, step) : team_sync(t);
-                    if (!ok) {
-                        stage_drain(st);
-                        return;
-                    }
+                    bool ok;
+                    if (handoff && !last) ok = step_handoff(p, t, step);
+                    else if (team_sync_or(t, !landed, ok)) ok = false;
+                    if (!ok) return stage_drain(st);
                     if (isLead) {
                         const unsigned long long tc = clock64();
                         cycRelax += tb - ta;
@@ -1119,7 +1123,7 @@ __device__ __forceinline__ void bf_run(const BfParams& p, const Team& t, char* s
         }
         if (stop) {
             if (isLead) { p.ctl->status = BF_LAYER_UNREACHED; p.ctl->sweeps = sweep; p.ctl->epoch = epochBase + sweep; }
-            return;
+            return true;
         }
         if (p.mode == 1) {
             if (isLead) {
@@ -1127,7 +1131,7 @@ __device__ __forceinline__ void bf_run(const BfParams& p, const Team& t, char* s
                 p.ctl->sweeps = sweep;
                 p.ctl->epoch = epochBase + sweep;
             }
-            return;
+            return true;
         }
         const size_t lastRowBase = (size_t)lastPar * n * Kp + lastDepth;
         if (p.mode == 2) {
@@ -1158,7 +1162,7 @@ __device__ __forceinline__ void bf_run(const BfParams& p, const Team& t, char* s
                 p.redIdx[2 * t.cta + 1] = firstValid.i;
                 p.redAux[t.cta] = anyFinite;
             }
-            if (!team_sync(t)) return;
+            if (!team_sync(t)) return true;
             if (isLead) {
                 Key f{kInfD, 0x7fffffff}, fv{kInfD, 0x7fffffff};
                 int af = 0;
@@ -1179,7 +1183,7 @@ __device__ __forceinline__ void bf_run(const BfParams& p, const Team& t, char* s
                 p.ctl->sweeps = sweep;
                 p.ctl->epoch = epochBase + sweep;
             }
-            return;
+            return true;
         }
 
         // wrap-around (cost_time_ratio_solver.cpp:399-417) and lap function
@@ -1220,10 +1224,10 @@ __device__ __forceinline__ void bf_run(const BfParams& p, const Team& t, char* s
             bool ok;
             improved = team_sync_or(t, improved, ok);
             if (isLead) atomicAdd(&p.ctl->cycWrap, clock64() - tTail);
-            if (!ok) return;
+            if (!ok) return true;
             if (!improved) {
                 if (isLead) { p.ctl->status = BF_WRAP_NO_IMPROVE; p.ctl->sweeps = sweep; p.ctl->epoch = epochBase + sweep; }
-                return;
+                return true;
             }
         }
 
@@ -1270,7 +1274,7 @@ __device__ __forceinline__ void bf_run(const BfParams& p, const Team& t, char* s
         __shared__ long long sCycLen;
         __shared__ Key sOk, sUnk;
         const unsigned long long tCand = isLead ? clock64() : 0;
-        if (!team_sync(t)) return;
+        if (!team_sync(t)) return true;
         // Every CTA reads the team's best decided candidate and its first
         // undecided one.  Undecided candidates that precede the best decided
         // one are walked literally, all at once, in bounded rounds; then the
@@ -1310,7 +1314,7 @@ __device__ __forceinline__ void bf_run(const BfParams& p, const Team& t, char* s
                     if (__ldcg(p.candStat + i) == 3 && !walk_advance(p, (int)i, kWalkRoundLoads)) pending = 1;
                 bool good;
                 pending = team_sync_or(t, pending, good);
-                if (!good) return;
+                if (!good) return true;
                 if (isLead) p.ctl->walkRounds = round + 1;
                 if (!pending) break;
             }
@@ -1325,7 +1329,7 @@ __device__ __forceinline__ void bf_run(const BfParams& p, const Team& t, char* s
                 p.redVal[2 * t.cta] = best.v;
                 p.redIdx[2 * t.cta] = best.i;
             }
-            if (!team_sync(t)) return;
+            if (!team_sync(t)) return true;
             if (isLead) {
                 ok = Key{kInfD, 0x7fffffff};
                 for (int c = 0; c < t.ncta; ++c) {
@@ -1401,16 +1405,18 @@ __device__ __forceinline__ void bf_run(const BfParams& p, const Team& t, char* s
         bool tailOk;
         finished = team_sync_or(t, finished, tailOk);
         if (isLead) atomicAdd(&p.ctl->cycTail, clock64() - tTail);
-        if (!tailOk || finished) return;
+        if (!tailOk || finished) return true;
     }
 }
 
 // bf_run between the two mbarriers' first and last use: it initialises them
 // (with the CTA's lists or tables) and leaves them at one point of the code for
 // the whole CTA; they are given up here, so that the next call of the launch
-// finds plain memory.
+// finds plain memory.  False when bf_run's waits for a copy, the last one
+// included, ran out: the copy may still write the CTA's shared memory, and the
+// CTA must use it no more.
 template <class CT, int TK, bool S, int SITE = 0>
-__device__ __forceinline__ void bf_body(const BfParams& p, const Team& t, char* smem) {
+__device__ __forceinline__ bool bf_body(const BfParams& p, const Team& t, char* smem) {
     unsigned long long* bar;
     if constexpr (SITE > 0) {
         bar = local_hot().bar;
@@ -1418,13 +1424,14 @@ __device__ __forceinline__ void bf_body(const BfParams& p, const Team& t, char* 
         __shared__ unsigned long long stageBar[2];
         bar = stageBar;
     }
-    bf_run<CT, TK, S, SITE>(p, t, smem, bar);
+    if (!bf_run<CT, TK, S, SITE>(p, t, smem, bar)) return false;
     __syncthreads();
     if (threadIdx.x == 0) {
         mbar_inval(bar);
         mbar_inval(bar + 1);
     }
     __syncthreads();
+    return true;
 }
 
 // The Bellman-Ford launch of one graph.  Every CTA of the grid belongs to
@@ -1725,27 +1732,34 @@ __device__ int record_cycle(const PairJob& J, const BfParams& P, const Team& t, 
 }
 
 template <class CT, int TK>
-__device__ __noinline__ void bf_call(const BfParams& P, const Team& t) {
-    bf_body<CT, TK, false>(P, t, reinterpret_cast<char*>(smemRaw));
+__device__ __noinline__ bool bf_call(const BfParams& P, const Team& t) {
+    return bf_body<CT, TK, false>(P, t, reinterpret_cast<char*>(smemRaw));
 }
 template <class CT, int TK>
-__device__ __forceinline__ void bf_local_call(const BfParams& P, const Team& t) {
-    bf_body<CT, TK, false, 2>(P, t, nullptr);
+__device__ __forceinline__ bool bf_local_call(const BfParams& P, const Team& t) {
+    return bf_body<CT, TK, false, 2>(P, t, nullptr);
 }
 
 // One Bellman-Ford call of the team: the lead publishes the call's state,
 // the Bellman-Ford CTAs run it, and every CTA reads its verdict after the
-// closing barrier.  False when a team barrier ran out.
+// closing barrier.  False when a team barrier ran out, or when this CTA left
+// copies in flight (`lost`): then it raises the team's error word, and the
+// others give up at that barrier, which it never reaches.
 template <class CT, int TK>
-__device__ __forceinline__ bool team_bf_call(PairJob& J, const BfParams& P, const SolveTeam& S, bool resetError) {
+__device__ __forceinline__ bool team_bf_call(PairJob& J, const BfParams& P, const SolveTeam& S, bool resetError,
+                                             bool& lost) {
     if (S.lead()) {
         P.ctl->status = BF_RUNNING;
         if (resetError) P.ctl->error = 0;
     }
     if (!team_sync(S.all)) return false;
     if (S.in_bf()) {
-        if (P.localKD) bf_local_call<CT, TK>(P, S.bf);
-        else bf_call<CT, TK>(P, S.bf);
+        if (P.localKD) lost = !bf_local_call<CT, TK>(P, S.bf);
+        else lost = !bf_call<CT, TK>(P, S.bf);
+        if (lost) {
+            if (threadIdx.x == 0) atomicExch(S.all.err, 1);
+            return false;
+        }
     }
     if (!team_sync(S.all)) return false;
     if (S.lead()) {
@@ -1759,19 +1773,21 @@ __device__ __forceinline__ bool team_bf_call(PairJob& J, const BfParams& P, cons
 // Bellman-Ford parameters in each CTA's shared memory.  Work over nodes and
 // cycle edges is spread over the team's threads; the sums over a cycle run on
 // one thread of every CTA, in the same order, so every CTA takes the same
-// branches; only the lead writes the job's outputs.
+// branches; only the lead writes the job's outputs.  False: the CTA may take no
+// further job (its shared memory may still be written).
 template <class CT, int TK>
-__device__ __forceinline__ void pair_solve(PairJob& J, BfParams& P, const SolveTeam& S) {
+__device__ __forceinline__ bool pair_solve(PairJob& J, BfParams& P, const SolveTeam& S) {
     const Team& t = S.all;
     const bool lead = S.lead();
     const int n = P.n;
     Control* ctl = P.ctl;
+    bool lost = false;
     const double tolerance = (double)(float)1e-8;
     const double ubInf = (double)__int_as_float(0x7f800000);
 #define PGC_TEAM_FAIL()                                \
     do {                                               \
         if (lead) J.status = PAIR_ERR_WAIT;            \
-        return;                                        \
+        return !lost;                                  \
     } while (0)
 
     // ---- initial upper bound (cost_time_ratio_solver.cpp:652-707) ----
@@ -1834,27 +1850,27 @@ __device__ __forceinline__ void pair_solve(PairJob& J, BfParams& P, const SolveT
             P.lambda = currentRatio;
             P.ub = ubInf;
         }
-        if (!team_bf_call<CT, TK>(J, P, S, search)) PGC_TEAM_FAIL();
+        if (!team_bf_call<CT, TK>(J, P, S, search, lost)) PGC_TEAM_FAIL();
         if (lead && !search) J.lawlerIters++;
         if (*(volatile int*)&ctl->error) PGC_TEAM_FAIL();
         const int st = *(volatile int*)&ctl->status;
         if (search) {
             if (st == BF_LAYER_UNREACHED) {  // the empty cycle's 0/0 bound: (true, NaN, no rows)
                 if (lead) J.status = PAIR_NAN;
-                return;
+                return true;
             }
             if (st != BF_UB_DONE) {
                 if (lead) {
                     J.status = st < 0 ? PAIR_ERR_BF : PAIR_ERR_UB;
                     J.bfStatus = st;
                 }
-                return;
+                return true;
             }
             const int m = record_cycle(J, P, t, neg, *(volatile int*)&ctl->cycleLen, false);
             if (m == -3) PGC_TEAM_FAIL();
             if (m < 0) {
                 if (lead) J.status = m == -2 ? PAIR_HOST : PAIR_ERR_EDGE;
-                return;
+                return true;
             }
             negEdges = m;
             double lambda = 10;
@@ -1862,7 +1878,7 @@ __device__ __forceinline__ void pair_solve(PairJob& J, BfParams& P, const SolveT
             for (int guard = 0; via_float(ev.wsum) > 0 || isnan(via_float(ev.wsum));) {
                 if (++guard > 4000) {
                     if (lead) J.status = PAIR_ERR_GUARD;
-                    return;
+                    return true;
                 }
                 lambda += lambda;
                 ev = record_sums(J, neg, m, lambda);
@@ -1872,7 +1888,7 @@ __device__ __forceinline__ void pair_solve(PairJob& J, BfParams& P, const SolveT
             // heap comparison that ends the first branch does not hold then).
             if (!(bound < (double)__int_as_float(0x7f800000))) {
                 if (lead) J.status = PAIR_HOST;
-                return;
+                return true;
             }
             for (long long v = t.thread(); v < n; v += t.nthreads()) J.branchOf[v] = 0;
             currentRatio = oldRatio = bound;
@@ -1887,7 +1903,7 @@ __device__ __forceinline__ void pair_solve(PairJob& J, BfParams& P, const SolveT
             if (m == -3) PGC_TEAM_FAIL();
             if (m < 0) {
                 if (lead) J.status = m == -2 ? PAIR_HOST : PAIR_ERR_EDGE;
-                return;
+                return true;
             }
             const CycleSums ev = record_sums(J, cand, m, currentRatio);
             if (round_to_int_x86(ev.wsum) >= 0) break;
@@ -1901,7 +1917,7 @@ __device__ __forceinline__ void pair_solve(PairJob& J, BfParams& P, const SolveT
                 J.status = PAIR_ERR_BF;
                 J.bfStatus = st;
             }
-            return;
+            return true;
         }
         // lawlerSoubroutine's update and stopping rules (:584-597)
         currentRatio = sums.ratio;
@@ -1914,7 +1930,7 @@ __device__ __forceinline__ void pair_solve(PairJob& J, BfParams& P, const SolveT
     const CycleSums fin = record_sums(J, neg, negEdges, currentRatio);
     // passes of the cycle through layer 0 (:606-634): more than one, and the
     // branch and bound splits the branch -- the host's part
-    if (t.cta != 0) return;
+    if (t.cta != 0) return true;
     __shared__ int sWraps;
     if (threadIdx.x == 0) sWraps = 0;
     __syncthreads();
@@ -1943,6 +1959,7 @@ __device__ __forceinline__ void pair_solve(PairJob& J, BfParams& P, const SolveT
             J.status = PAIR_DONE;
         }
     }
+    return true;
 #undef PGC_TEAM_FAIL
 }
 
@@ -1976,7 +1993,7 @@ __global__ void __launch_bounds__(kBatchThreads, 1)
         __syncthreads();
         const SolveTeam S{all, Team{cta, sCtas, &P.ctl->barCount, &P.ctl->barGen, &P.ctl->error, P.spinLimit}};
         const long long c0 = clock64();
-        pair_solve<CT, TK>(jobs[j], P, S);
+        if (!pair_solve<CT, TK>(jobs[j], P, S)) return;
         if (lead) {
             jobs[j].candidates = P.ctl->candidates;
             jobs[j].fallbackWalks = P.ctl->fallbackWalks;

@@ -1222,12 +1222,14 @@ BfParams Graph::params(const Run& r, int mode, int branchId, double lambda, doub
     p.mode = mode;
     p.maxSweeps = 0;
     // device waits give up after this many polls (PGC_BF_SPIN_LIMIT: tests
-    // of the timeout path use a short one); two test hooks, off in every
+    // of the timeout path use a short one); three test hooks, off in every
     // solve: PGC_BF_TEST_STALL_CTA makes that CTA's step hand-off also wait
-    // for a word no code writes, and PGC_BF_LITERAL_WALKS=1 decides every
-    // candidate by the literal predecessor walk
+    // for a word no code writes, PGC_BF_TEST_STALL_COPY makes that CTA's waits
+    // for staged copies run out at once, and PGC_BF_LITERAL_WALKS=1 decides
+    // every candidate by the literal predecessor walk
     p.spinLimit = (unsigned)std::max(1, env_int("PGC_BF_SPIN_LIMIT", (int)kDefaultSpinLimit));
     p.stallCta = env_int("PGC_BF_TEST_STALL_CTA", -1);
+    p.stallCopyCta = env_int("PGC_BF_TEST_STALL_COPY", -1);
     p.literalAll = env_int("PGC_BF_LITERAL_WALKS", 0) ? 1 : 0;
     p.ctl = wCtl.p;
     p.cycleBuf = wCycle.p;
@@ -1828,6 +1830,7 @@ void Graph::finish_job(const PairJob& J, int K) {
             solve_ratio_rescaled(K, &first);
             return;
         }
+        case PAIR_PENDING:  // its team gave up on an earlier graph of the batch
         case PAIR_ERR_WAIT:
             wLayerFlag.zero(stream);
             ctlEpoch = 0;
