@@ -15,8 +15,11 @@
 // number tells whether the value beside it is the one waited for: no fence,
 // no flag and no barrier lie between a node's store and its readers' polls.
 // Two parities of records exist per depth; a CTA overwrites one only after
-// every neighbour has reported (stepDone) that it read the record before it,
-// two layers back.
+// every neighbour has reported that it read the record before it, two layers
+// back.  That report does need an order: stepDone is published with release
+// and polled with acquire semantics, a CTA barrier on either side, so that a
+// neighbour's read comes before the store that replaces what it read.  Both are
+// the staging warp's, off the path of the relaxing ones.
 //
 // What it replaces: sources gathered from L2 per in-edge, and a release /
 // acquire hand-off of per-CTA step counters with two CTA barriers around it
@@ -58,15 +61,6 @@ __device__ __forceinline__ void ld_record(const uint4* at, double& v, unsigned& 
     tag = (unsigned)hi;
     oh = (unsigned)(hi >> 32);
 }
-__device__ __forceinline__ unsigned ld_relaxed_u32(const unsigned* p) {
-    unsigned v;
-    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_relaxed_u32(unsigned* p, unsigned v) {
-    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
 // gid word of an own table entry: its node, bit 30 when another CTA reads it;
 // negative where the slot holds no node.  Of a halo entry: its node.
 constexpr int kGidExposed = 1 << 30;
@@ -652,7 +646,7 @@ __device__ __noinline__ unsigned local_sweep(int stamp, unsigned step, unsigned 
                                 i < nWait ? H.stepDone + (size_t)__ldg(H.waitIdx + i) * kStepDoneStride : H.neverSet;
                             const int want = i < nWait ? (int)step + 1 - 2 * KD : (int)step;
                             unsigned spins = 0;
-                            while ((int)ld_relaxed_u32(f) < want)
+                            while ((int)ld_acquire_u32(f) < want)
                                 if (local_give_up(H, step, spins)) break;
                         }
                     }
@@ -660,7 +654,10 @@ __device__ __noinline__ unsigned local_sweep(int stamp, unsigned step, unsigned 
                     if (lane == 0 && H.cta == 0) H.cyc[2] += (unsigned)clock() - t0;
                 }
                 __syncthreads();
-                if (lane == 0 && H.ncta > 1) st_relaxed_u32(H.stepDone + (size_t)H.cta * kStepDoneStride, step);
+                // release: the halo reads of the CTA's threads, before the
+                // barrier, come before what the neighbours store after they
+                // have seen this
+                if (lane == 0 && H.ncta > 1) st_release_u32(H.stepDone + (size_t)H.cta * kStepDoneStride, step);
                 sb ^= 1;
                 stopped = H.stop[step & 3];
             }

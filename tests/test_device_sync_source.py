@@ -48,3 +48,17 @@ def test_a_cta_leaves_a_step_as_one(functions):
     assert re.search(r"if \(threadIdx\.x == 0\) \{[^{}]*sGood = [^;]*t\.err[^;]*;\s*\}", body)
     assert "__any_sync(0xffffffffu, (spins & 63u) == 0 && *(volatile int*)t.err)" in body
     assert body.count("t.err") == body.count("atomicExch(t.err, 1)") + 2
+
+
+def test_exchanged_records_are_overwritten_after_their_reads(functions):
+    """A CTA's report that it has read its neighbours' records (stepDone) is
+    the only order between those reads and the stores that replace the records:
+    release and acquire, each beyond a CTA barrier."""
+    body = functions["local_sweep"]
+    assert re.search(r"__syncthreads\(\);\s*if \(lane == 0 && H\.ncta > 1\) st_release_u32\(H\.stepDone", body)
+    assert "while ((int)ld_acquire_u32(f) < want)" in body
+    assert len(re.findall(r"H\.stepDone", body)) == 2
+    for f, b in functions.items():
+        assert "relaxed.gpu.global.u32" not in b, f
+    assert "st.release.gpu.global.u32" in functions["st_release_u32"]
+    assert "ld.acquire.gpu.global.u32" in functions["ld_acquire_u32"]
