@@ -33,6 +33,7 @@ def test_stalled_copy_ends_the_solve(cpg, oracle, monkeypatch, local, blocks, ct
     g, o = cpg.product_graph_generator(*args), oracle.OracleGenerator(*args)
     monkeypatch.setenv("PGC_BF_LOCAL", local)
     monkeypatch.setenv("PGC_BF_BLOCKS", blocks)
+    monkeypatch.setenv("PGC_BF_THREADS", "64")  # two warps a CTA: CTA 5 of 8 has slices in both layouts
     monkeypatch.setenv("PGC_BF_TEST_STALL_COPY", cta)
     for solve, name in ((g.solve_with_cost_time_ratio, "lawlergpu"), (g.solve_with_minimum_cost, "dijkstragpu")):
         t0 = time.perf_counter()
