@@ -199,6 +199,11 @@ int pgc_solve_batch(pgc_graph* const* graphs, int64_t count, const char* solver_
  * process so far, on every device and thread (a counter that only grows). */
 int pgc_kernel_launches(int64_t* out);
 
+/* No reference counterpart.  How often this process has built and uploaded the
+ * node ranges and wait lists of a Bellman-Ford team: once per handle and team
+ * shape that follows another one, not once per solve. */
+int pgc_team_uploads(int64_t* out);
+
 /* No reference counterpart.  Where the calling thread's last
  * pgc_solve_batch spent its time (host wall clock, ms) when it solved ratio
  * cycles in one launch: out8 = {costs generated and rescaled, teams

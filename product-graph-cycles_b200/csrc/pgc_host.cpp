@@ -507,10 +507,10 @@ class Graph {
         double bound, lambda;
         CycleRec cycle;
     };
-    void solve_ratio_rescaled(int K, const FirstBranch* first = nullptr);
-    bool solve_ratio_device(int K);
+    void solve_ratio_rescaled(const Run& r, const FirstBranch* first = nullptr);
+    void solve_ratio_device(const Run& r);
     void fill_job(const Run& r, PairJob& J);
-    void finish_job(const PairJob& J, int K);
+    void finish_job(const PairJob& J, int K, const Run* r);
     DBuf<PairJob> wJob;
     DBuf<unsigned> wJobWords;  // the team's barrier words, then the queue's counter
     void ensure_workspace(int K, int blocks);
@@ -1055,8 +1055,6 @@ bool Graph::plan_local(Run& r, int blocks, size_t smemCap) {
         }
         q.parts = parts;
         q.cut = cut;
-    } else {
-        upload_cta_slices(cut, r.K, -1);
     }
     if (!q.fits) return false;
     const int costBytes = r.costF32 ? 4 : 8, timeBytes = r.timeKind == 1 ? 4 : r.timeKind == 2 ? 8 : 0;
@@ -1069,6 +1067,9 @@ bool Graph::plan_local(Run& r, int blocks, size_t smemCap) {
         if (tables > smemCap) return false;
     }
     if (blocks > 1) wXbuf.alloc((size_t)2 * KD * nslots);
+    // only here: a graph that goes on to the sweeps in global memory keeps
+    // the ranges and wait lists that those uploaded last
+    upload_cta_slices(cut, r.K, -1);
     r.localKD = KD;
     r.hopBits = hopBits;
     r.blocks = blocks;
@@ -1078,6 +1079,10 @@ bool Graph::plan_local(Run& r, int blocks, size_t smemCap) {
     r.stageSrcOnly = 0;
     return true;
 }
+
+// CTA ranges and wait lists built and uploaded by this process
+// (pgc_team_uploads).
+std::atomic<long long> g_teamUploads{0};
 
 // CTA slice ranges of the team (plan_cta_cuts), cached per (blocks, K,
 // warps).  A warp gathers bf_rows_per_batch(K) interlayer rows per batch
@@ -1100,6 +1105,7 @@ std::vector<int> Graph::cta_cuts(int blocks, int K, int warps) const {
 void Graph::upload_cta_slices(const std::vector<int>& cut, int K, int warps) {
     const int blocks = (int)cut.size() - 1;
     if (cutBlocks == blocks && cutK == K && cutWarps == warps && ctaCut == cut) return;
+    g_teamUploads.fetch_add(1, std::memory_order_relaxed);
     std::vector<int> ptr, idx;
     cta_wait_lists(T, cut, ptr, idx);
     wCtaSlice.upload(cut.data(), cut.size(), stream);
@@ -1387,16 +1393,16 @@ void Graph::solve_ratio(int K) {
     const double scaling = 100000.0;
     // In-place rescale of the generator's costs (cost_time_ratio_solver.cpp:875-882).
     rescale_columns(scaling);
-    if (!solve_ratio_device(K)) solve_ratio_rescaled(K);
+    const Run r = prepare_run(K, true);
+    if (r.localKD) solve_ratio_device(r);
+    else solve_ratio_rescaled(r);
 }
 
 // The ratio solve by one launch of the batched solver with this graph alone:
 // its whole team runs the upper bound, the Lawler iterations and the cycle
 // evaluations on the device, where the host-driven solve waits twice per
-// Bellman-Ford call.  False: the graph's team does not run on local tables.
-bool Graph::solve_ratio_device(int K) {
-    const Run r = prepare_run(K, true);
-    if (!r.localKD) return false;
+// Bellman-Ford call.  For teams on local tables.
+void Graph::solve_ratio_device(const Run& r) {
     reset_predecessors();
     PairJob J;
     fill_job(r, J);
@@ -1418,21 +1424,19 @@ bool Graph::solve_ratio_device(int K) {
     PGC_CUDA(sync_stream());
     float ms = 0;
     cudaEventElapsedTime(&ms, timeEvents[0], timeEvents[1]);
-    finish_job(J, K);
+    finish_job(J, r.K, &r);
     if (J.status != PAIR_HOST) {
         stats.deviceMs += ms;
         stats.launches += launches + 1;
     }
-    return true;
 }
 
 // The ratio solve after the rescale: the initial upper bound, then branch
 // and bound with Lawler in each branch (cost_time_ratio_solver.cpp:741-864).
 // `first`: the bound and the first branch's Lawler are done already; what is
 // left starts from that branch's cycle.
-void Graph::solve_ratio_rescaled(int K, const FirstBranch* first) {
+void Graph::solve_ratio_rescaled(const Run& r, const FirstBranch* first) {
     const double scaling = 100000.0;
-    Run r = prepare_run(K, true);
     if (!first) reset_predecessors();
     const int n = T.n;
     const long long nn = numNodes();
@@ -1751,7 +1755,7 @@ void Graph::batch_end(const PairJob& J, int ctas) {
         ~Cap() { cap = saved; }
     } restore{teamCap, teamCap};
     if (ctas > 0) teamCap = ctas;
-    finish_job(J, batchK);
+    finish_job(J, batchK, nullptr);
     if (J.status != PAIR_HOST) {
         stats.launches += launches;
         DeviceInfo info{};
@@ -1761,9 +1765,10 @@ void Graph::batch_end(const PairJob& J, int ctas) {
 }
 
 // The result from a finished job, or the solve finished on the host when the
-// device handed it back; statistics of the solve but for its launches and its
-// device time.
-void Graph::finish_job(const PairJob& J, int K) {
+// device handed it back, by the team that `r` prepared or, without one (a
+// batch's team is not a single solve's), by one prepared here; statistics of
+// the solve but for its launches and its device time.
+void Graph::finish_job(const PairJob& J, int K, const Run* r) {
     stats = Stats();
     Control c{};
     d2h(&c, wCtl.p, sizeof(Control));
@@ -1813,7 +1818,7 @@ void Graph::finish_job(const PairJob& J, int K) {
             // branch and bound (or a cycle longer than the device record):
             // the host's solve from the rescaled costs
             stats = Stats();
-            solve_ratio_rescaled(K);
+            solve_ratio_rescaled(r ? *r : prepare_run(K, true));
             return;
         case PAIR_WRAPS: {
             FirstBranch first{J.bound, J.lambda, {}};
@@ -1827,7 +1832,7 @@ void Graph::finish_job(const PairJob& J, int K) {
             d2h(first.cycle.c.data(), bRecC[J.rec].p, sizeof(double) * m);
             d2h(first.cycle.t.data(), bRecT[J.rec].p, sizeof(double) * m);
             PGC_CUDA(sync_stream());
-            solve_ratio_rescaled(K, &first);
+            solve_ratio_rescaled(r ? *r : prepare_run(K, true), &first);
             return;
         }
         case PAIR_PENDING:  // its team gave up on an earlier graph of the batch
@@ -2604,6 +2609,13 @@ int pgc_kernel_launches(int64_t* out) {
     return guarded([&] {
         if (!out) throw Failure(PGC_ERR_ARG, "null output");
         *out = pgc::launch_count();
+    });
+}
+
+int pgc_team_uploads(int64_t* out) {
+    return guarded([&] {
+        if (!out) throw Failure(PGC_ERR_ARG, "null output");
+        *out = pgc::g_teamUploads.load();
     });
 }
 

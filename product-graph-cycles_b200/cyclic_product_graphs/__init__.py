@@ -85,6 +85,7 @@ def _declare(L):
     L.pgc_device_name.argtypes = [_h, ctypes.c_char_p, _i64]
     L.pgc_batch_profile.argtypes = [_dp]
     L.pgc_kernel_launches.argtypes = [_lp]
+    L.pgc_team_uploads.argtypes = [_lp]
     L.pgc_last_error.restype = ctypes.c_char_p
     L.pgc_version.restype = ctypes.c_char_p
 
