@@ -429,6 +429,12 @@ cudaError_t launch_median_rescale(const SelectArgs& a, unsigned long long* topHi
 cudaError_t launch_rescale_f64(const SelectArgs& a, MedianState* st, double clip, cudaStream_t s);
 cudaError_t launch_to_f64(const float* col32, double* col, const StreamView& view, cudaStream_t s);
 cudaError_t launch_to_f32(const double* col, float* col32, const StreamView& view, int* exact, cudaStream_t s);
+// A column's streams in another order of the layer's entries: entry i of a
+// layer of `out` is entry from[i] of that layer of `in`, NaN where from[i] < 0.
+cudaError_t launch_reorder(const float* in, float* out, const int* from, long long inStride, long long outStride,
+                           int layers, cudaStream_t s);
+cudaError_t launch_reorder(const double* in, double* out, const int* from, long long inStride, long long outStride,
+                           int layers, cudaStream_t s);
 cudaError_t launch_row_masks(const int* tedge, long long entries, unsigned* mask, cudaStream_t s);
 cudaError_t launch_export(const double* col, double* out, int cols, int c, long long total, long long layerStride,
                           long long interEntries, int nY, long long eBlock, const int* ti, const int* tr,

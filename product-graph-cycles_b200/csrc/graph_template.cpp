@@ -609,6 +609,21 @@ std::vector<int> plan_even_cuts(const LayerTemplate& T, int blocks, int K) {
     return cut;
 }
 
+std::vector<int> stream_positions(const LayerTemplate& from, const LayerTemplate& to) {
+    std::vector<int> at((size_t)from.eBlock, -1), out((size_t)to.layerStride(), -1);
+    int base = 0;
+    for (int p = 0; p < 2; ++p) {
+        for (int64_t q = 0; q < from.entries[p]; ++q)
+            if (from.tedge[p][(size_t)q] >= 0) at[(size_t)from.tedge[p][(size_t)q]] = base + (int)q;
+        base += (int)from.entries[p];
+    }
+    size_t i = 0;
+    for (int p = 0; p < 2; ++p)
+        for (int64_t q = 0; q < to.entries[p]; ++q, ++i)
+            if (to.tedge[p][(size_t)q] >= 0) out[i] = at[(size_t)to.tedge[p][(size_t)q]];
+    return out;
+}
+
 // Wait lists of the Bellman-Ford team in CSR form (ptr: blocks + 1 offsets,
 // idx: CTA ids, ascending per list): CTA c lists every other CTA d joined to
 // it by an in-edge of either part, i.e. d owns the slice of a source of one

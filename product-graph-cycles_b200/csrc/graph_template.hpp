@@ -110,6 +110,11 @@ struct LayerTemplate {
 std::string build_template(const int* EX, int64_t nEX, const int* EY, int64_t nEY, int64_t nVX, bool conj,
                            bool prune, LayerTemplate& T, bool meshOrder = false);
 
+// For every entry of a layer's streams in the order of `to`, interlayer part
+// first, the entry of `from` that holds the same template edge; -1 where `to`
+// holds none.  Two templates of one graph in different orders.
+std::vector<int> stream_positions(const LayerTemplate& from, const LayerTemplate& to);
+
 // Runs f(begin, end) over parts of [0, n) of at least `grain` items on the
 // process's host worker pool (inline when another job holds the pool).
 void host_parallel_for(int64_t n, int64_t grain, const std::function<void(int64_t, int64_t)>& f);

@@ -90,6 +90,20 @@ __global__ void row_mask_kernel(const int* tedge, long long entries, unsigned* m
     }
 }
 
+// One thread per entry and chunk of kReorderLayers layers: its source entry is
+// read once, and a warp's stores are 32 consecutive entries of one layer.
+constexpr int kReorderLayers = 8;
+template <class CT>
+__global__ void reorder_kernel(const CT* in, CT* out, const int* from, long long inStride, long long outStride,
+                               int layers) {
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i >= outStride) return;
+    const int f = __ldg(from + i);
+    const int l0 = (int)blockIdx.y * kReorderLayers, l1 = min(l0 + kReorderLayers, layers);
+    const CT nan = (CT)__int_as_float(0x7fc00000);
+    for (int l = l0; l < l1; ++l) out[l * outStride + i] = f >= 0 ? __ldg(in + l * inStride + f) : nan;
+}
+
 // Order-preserving 64-bit image of a double (the median selection's keys).
 __device__ __forceinline__ unsigned long long order_key(double x) {
     const unsigned long long u = (unsigned long long)__double_as_longlong(x);
@@ -1613,6 +1627,26 @@ cudaError_t launch_to_f32(const double* col, float* col32, const StreamView& vie
     note_launch();
     to_f32_kernel<<<stream_grid(to_f32_kernel, 256, 0), 256, 0, s>>>(col, col32, view, exact);
     return cudaGetLastError();
+}
+template <class CT>
+static cudaError_t reorder(const CT* in, CT* out, const int* from, long long inStride, long long outStride, int layers,
+                           cudaStream_t s) {
+    // grids of at most 65,535 layer chunks
+    for (int l0 = 0; l0 < layers; l0 += 65535 * kReorderLayers) {
+        const int m = std::min(layers - l0, 65535 * kReorderLayers);
+        const dim3 grid((unsigned)((outStride + 255) / 256), (unsigned)((m + kReorderLayers - 1) / kReorderLayers));
+        note_launch();
+        reorder_kernel<CT><<<grid, 256, 0, s>>>(in + l0 * inStride, out + l0 * outStride, from, inStride, outStride, m);
+    }
+    return cudaGetLastError();
+}
+cudaError_t launch_reorder(const float* in, float* out, const int* from, long long inStride, long long outStride,
+                           int layers, cudaStream_t s) {
+    return reorder(in, out, from, inStride, outStride, layers, s);
+}
+cudaError_t launch_reorder(const double* in, double* out, const int* from, long long inStride, long long outStride,
+                           int layers, cudaStream_t s) {
+    return reorder(in, out, from, inStride, outStride, layers, s);
 }
 cudaError_t launch_row_masks(const int* tedge, long long entries, unsigned* mask, cudaStream_t s) {
     if (entries == 0) return cudaSuccess;

@@ -451,6 +451,7 @@ class Graph {
     void batch_end(const PairJob& job, int ctas);
     int batchK = 0;
     size_t batchSmem = 0;  // dynamic shared memory the prepared batch team needs
+    int batchCostF32 = 0, batchTimeKind = 0;  // its streams' types
     size_t batch_smem_bytes() const { return batchSmem; }
     DBuf<int> bRecNodes[2];
     DBuf<long long> bRecEdges[2];
@@ -479,10 +480,28 @@ class Graph {
         int rowCap;         // rows a step buffer holds (0: streams read in place)
         int stageSrcOnly;   // the buffers hold source indices only
         int localKD;        // depths of the per-CTA local tables (0: records in global memory)
+        bool byNode;        // lists and streams of nodeLists instead of the template's
         int hopBits;
         size_t smemBytes;   // dynamic shared memory per CTA
     };
     Run prepare_run(int K, bool ratio);
+    // The in-edge lists by node id, with the streams in their order: what a
+    // plain graph's sweeps in global memory read.  Their records and
+    // predecessors lie by node id; with the slots of a slice along the mesh
+    // the stores of a warp went to 32 sectors each, and a step of a 2,000 x
+    // 100 pair at K = 5 took 13.6k cycles instead of 11.0k.  A conjugate
+    // graph's sweeps gain more from slices of one kind and width than that
+    // costs (14,000 x 100, K = 3: 24.1k cycles a step by node id, 20.1k along
+    // the mesh) and keep the template's.
+    struct NodeLists {
+        LayerTemplate T;
+        DBuf<int> sp[2], src[2], srcDummy, slots, from;
+        DBuf<float> f32[2];
+        DBuf<double> f64[2];
+        bool ready = false;
+    } nodeLists;
+    void take_node_lists(Run& r);
+    const LayerTemplate& lists(const Run& r) const { return r.byNode ? nodeLists.T : T; }
     bool plan_local(Run& r, int blocks, size_t smemCap);
     // the local tables' plan of the partition in ctaCut (local_plan_kernel)
     struct LocalPlan {
@@ -514,8 +533,8 @@ class Graph {
     DBuf<PairJob> wJob;
     DBuf<unsigned> wJobWords;  // the team's barrier words, then the queue's counter
     void ensure_workspace(int K, int blocks);
-    std::vector<int> cta_cuts(int blocks, int K, int warps) const;
-    void upload_cta_slices(const std::vector<int>& cut, int K, int warps);
+    std::vector<int> cta_cuts(const LayerTemplate& T, int blocks, int K, int warps) const;
+    void upload_cta_slices(const LayerTemplate& T, const std::vector<int>& cut, int K, int warps);
     void upload_branch(const std::vector<int>& branchOf);
     // Every solve starts from an unwritten predecessor table (-1), like the
     // reference's freshly allocated solver state.
@@ -836,7 +855,8 @@ Graph::Run Graph::prepare_run(int K, bool ratio) {
     const bool stageOn = env_int("PGC_BF_STAGE", 1) != 0;
     std::vector<int> cut;
     auto stage_need = [&](int blocks, int& maxSl, int& rowCap) -> size_t {
-        cut = cta_cuts(blocks, K, r.threads / 32);
+        const LayerTemplate& T = lists(r);
+        cut = cta_cuts(T, blocks, K, r.threads / 32);
         maxSl = 0;
         rowCap = 0;
         for (int c = 0; c < blocks; ++c) {
@@ -859,6 +879,7 @@ Graph::Run Graph::prepare_run(int K, bool ratio) {
             ensure_workspace(K, std::max(r.blocks, batchCtas));
             return r;
         }
+        if (!conj) take_node_lists(r);
         r.sharedTables = false;
         r.flagSync = r.blocks > 1 && env_int("PGC_BF_FLAGS", 1) ? 1 : 0;
         int maxSl = 0, rowCap = 0;
@@ -880,7 +901,7 @@ Graph::Run Graph::prepare_run(int K, bool ratio) {
         r.smemBytes = need;
         // the team's reductions outside the Bellman-Ford calls use every CTA
         ensure_workspace(K, std::max(r.blocks, batchCtas));
-        upload_cta_slices(cut, K, r.threads / 32);
+        upload_cta_slices(lists(r), cut, K, r.threads / 32);
         return r;
     }
     int envBlocks = env_int("PGC_BF_BLOCKS", 0), envThreads = env_int("PGC_BF_THREADS", 0);
@@ -920,6 +941,7 @@ Graph::Run Graph::prepare_run(int K, bool ratio) {
             return r;
         }
     }
+    if (!conj) take_node_lists(r);
     int maxSl = 0, rowCap = 0;
     int blocks = envBlocks;
     if (blocks <= 0 && T.nslices <= env_int("PGC_BF_SINGLE_CTA_SLICES", 64) &&
@@ -979,8 +1001,46 @@ Graph::Run Graph::prepare_run(int K, bool ratio) {
     r.flagSync = env_int("PGC_BF_FLAGS", 1) ? 1 : 0;
     ensure_workspace(K, blocks);
     if (cut.size() != (size_t)blocks + 1) stage_need(blocks, maxSl, rowCap);
-    upload_cta_slices(cut, K, r.threads / 32);
+    upload_cta_slices(lists(r), cut, K, r.threads / 32);
     return r;
+}
+
+// The run's lists and streams by node id: the lists once per handle, the
+// streams brought over on every run, since the costs may be new.
+void Graph::take_node_lists(Run& r) {
+    NodeLists& L = nodeLists;
+    if (!L.ready) {
+        const std::string err = build_template(EX.data(), nex, EY.data(), ney, nvx, conj, prune, L.T);
+        if (!err.empty()) throw Failure(PGC_ERR_ARG, err);
+        for (int p = 0; p < 2; ++p) {
+            L.sp[p].upload(L.T.sp[p].data(), L.T.sp[p].size(), stream);
+            L.src[p].upload(L.T.src[p].data(), L.T.src[p].size(), stream);
+        }
+        if (T.nY == 2) L.srcDummy.upload(L.T.srcDummy.data(), L.T.srcDummy.size(), stream);
+        std::vector<int> slots((size_t)L.T.nslices * 32, -1);
+        for (int v = 0; v < T.n; ++v) slots[(size_t)v] = v;
+        L.slots.upload(slots.data(), slots.size(), stream);
+        const std::vector<int> from = stream_positions(T, L.T);
+        L.from.upload(from.data(), from.size(), stream);
+        PGC_CUDA(sync_stream());
+        L.ready = true;
+    }
+    const long long in = T.layerStride(), out = L.T.layerStride();
+    auto bring = [&](const void* col, bool f32, int c) -> const void* {
+        const size_t total = (size_t)out * (T.nY + 1);
+        stats.launches++;
+        if (f32) {
+            L.f32[c].alloc(total);
+            PGC_CUDA(launch_reorder((const float*)col, L.f32[c].p, L.from.p, in, out, T.nY + 1, stream));
+            return L.f32[c].p;
+        }
+        L.f64[c].alloc(total);
+        PGC_CUDA(launch_reorder((const double*)col, L.f64[c].p, L.from.p, in, out, T.nY + 1, stream));
+        return L.f64[c].p;
+    };
+    r.cost = bring(r.cost, r.costF32 != 0, 0);
+    if (r.timeKind) r.time = bring(r.time, r.timeKind == 1, 1);
+    r.byNode = true;
 }
 
 // A team of `blocks` CTAs that sweeps on per-CTA local tables
@@ -1022,7 +1082,7 @@ bool Graph::plan_local(Run& r, int blocks, size_t smemCap) {
         wLocalCounts.alloc((size_t)2 * blocks);
         PGC_CUDA(cudaMemsetAsync(wExposed.p, 0, (size_t)T.nslices * 4, stream));
         PGC_CUDA(cudaMemsetAsync(wSliceUsed.p, 0, (size_t)T.nslices, stream));
-        upload_cta_slices(cut, r.K, -1);
+        upload_cta_slices(T, cut, r.K, -1);
         LocalPlanArgs a{};
         a.nslices = T.nslices;
         a.ncta = blocks;
@@ -1069,7 +1129,7 @@ bool Graph::plan_local(Run& r, int blocks, size_t smemCap) {
     if (blocks > 1) wXbuf.alloc((size_t)2 * KD * nslots);
     // only here: a graph that goes on to the sweeps in global memory keeps
     // the ranges and wait lists that those uploaded last
-    upload_cta_slices(cut, r.K, -1);
+    upload_cta_slices(T, cut, r.K, -1);
     r.localKD = KD;
     r.hopBits = hopBits;
     r.blocks = blocks;
@@ -1085,9 +1145,9 @@ bool Graph::plan_local(Run& r, int blocks, size_t smemCap) {
 std::atomic<long long> g_teamUploads{0};
 
 // CTA slice ranges of the team (plan_cta_cuts), cached per (blocks, K,
-// warps).  A warp gathers bf_rows_per_batch(K) interlayer rows per batch
+// warps); a handle's teams in global memory all have the same lists.  A warp gathers bf_rows_per_batch(K) interlayer rows per batch
 // (one row when K > 4) and bf_rows_per_batch(1) intralayer rows.
-std::vector<int> Graph::cta_cuts(int blocks, int K, int warps) const {
+std::vector<int> Graph::cta_cuts(const LayerTemplate& T, int blocks, int K, int warps) const {
     const std::string key = std::to_string(blocks) + "/" + std::to_string(K) + "/" + std::to_string(warps);
     {
         const auto it = cutCache.find(key);
@@ -1102,7 +1162,7 @@ std::vector<int> Graph::cta_cuts(int blocks, int K, int warps) const {
 // Uploads the slice range of every CTA (cta_cuts) and every CTA's wait list
 // (cta_wait_lists: the CTAs whose rows it reads through an in-edge, and the
 // CTAs that read its rows).
-void Graph::upload_cta_slices(const std::vector<int>& cut, int K, int warps) {
+void Graph::upload_cta_slices(const LayerTemplate& T, const std::vector<int>& cut, int K, int warps) {
     const int blocks = (int)cut.size() - 1;
     if (cutBlocks == blocks && cutK == K && cutWarps == warps && ctaCut == cut) return;
     g_teamUploads.fetch_add(1, std::memory_order_relaxed);
@@ -1172,8 +1232,6 @@ BfParams Graph::params(const Run& r, int mode, int branchId, double lambda, doub
     p.Kp = r.Kp;
     p.nslices = T.nslices;
     p.nslots = T.nslices * 32;
-    p.slotNode = dSlotNode.p;
-    p.nodeSlot = dNodeSlot.p;
     p.localKD = r.localKD;
     if (r.localKD) {
         p.localL = localPlan.L;
@@ -1191,14 +1249,19 @@ BfParams Graph::params(const Run& r, int mode, int branchId, double lambda, doub
         p.xbuf = wXbuf.p;
     }
     p.numNodes = numNodes();
-    p.spInter = dSp[INTER].p;
-    p.spIntra = dSp[INTRA].p;
-    p.srcInter = dSrc[INTER].p;
-    p.srcDummy = dSrcDummy.p ? dSrcDummy.p : dSrc[INTER].p;
-    p.srcIntra = dSrc[INTRA].p;
-    p.interEntries = T.entries[INTER];
-    p.intraEntries = T.entries[INTRA];
-    p.layerStride = T.layerStride();
+    const LayerTemplate& L = lists(r);
+    const DBuf<int>*sp = r.byNode ? nodeLists.sp : dSp, *src = r.byNode ? nodeLists.src : dSrc;
+    const DBuf<int>& dummy = r.byNode ? nodeLists.srcDummy : dSrcDummy;
+    p.slotNode = r.byNode ? nodeLists.slots.p : dSlotNode.p;
+    p.nodeSlot = r.byNode ? nodeLists.slots.p : dNodeSlot.p;
+    p.spInter = sp[INTER].p;
+    p.spIntra = sp[INTRA].p;
+    p.srcInter = src[INTER].p;
+    p.srcDummy = dummy.p ? dummy.p : src[INTER].p;
+    p.srcIntra = src[INTRA].p;
+    p.interEntries = L.entries[INTER];
+    p.intraEntries = L.entries[INTRA];
+    p.layerStride = L.layerStride();
     p.cost = r.cost;
     p.time = r.time;
     p.tconst = r.tconst;
@@ -1741,6 +1804,8 @@ void Graph::batch_begin(int K, PairJob& J, int threads, int ctas, size_t smemCap
     }
     batchThreads = 0;
     batchSmem = r.smemBytes;
+    batchCostF32 = r.costF32;
+    batchTimeKind = r.timeKind;
     reset_predecessors();
     fill_job(r, J);
     PGC_CUDA(sync_stream());
@@ -2711,9 +2776,8 @@ int pgc_solve_batch(pgc_graph* const* graphs, int64_t count, const char* solver,
                         throw;
                     }
                     g.blockingSync = false;
-                    costF32[(size_t)i] = jobs[(size_t)i].bf.cost == (const void*)g.e32[0].p ? 1 : 0;
-                    timeKind[(size_t)i] = jobs[(size_t)i].bf.time == nullptr ? 0
-                                          : jobs[(size_t)i].bf.time == (const void*)g.e32[1].p ? 1 : 2;
+                    costF32[(size_t)i] = g.batchCostF32;
+                    timeKind[(size_t)i] = g.batchTimeKind;
                     smemNeed[(size_t)i] = jobs[(size_t)i].bf.maxCtaSlices >= 0 ? g.batch_smem_bytes() : 0;
                     work[(size_t)i] = (double)g.T.layerStride() * g.T.nY * K;
                 });
