@@ -80,7 +80,7 @@ struct BfParams {
     // graph
     int n, nY, K, Kp, nslices, nslots;
     const int* slotNode;           // [nslots] target node of a list slot (32 * slice + lane), -1: none
-    const int* nodeSlot;           // [n] slot of a node
+    const int* nodeSlot;           // [n] slot of a node; both null: node v has slot v
     long long numNodes;            // n * nY
     const int* spInter;
     const int* spIntra;

@@ -179,10 +179,10 @@ __device__ __forceinline__ int original_index(int n, int K, int e) {
 // DP record of node v at depth k in the parity row starting at rowBase =
 // parity * n * Kp.  Its value lives in p.dv at rowBase + v * Kp + k (a
 // node's depths side by side: one vector load gathers them); its path origin
-// and length live in p.doh at rowBase + k * n + v (depth-major: the stores
-// of a warp's 32 consecutive nodes are 256 contiguous bytes, where the
-// node-major index would spread them over 32 sectors; they are read one at
-// a time).  Loads come from shared memory when the whole team is one CTA
+// and length live in p.doh at rowBase + k * n + v (depth-major: where slots
+// follow the node ids, as in a plain graph's sweeps here, the stores of a warp
+// are 256 contiguous bytes, which the node-major index would spread over 32
+// sectors; they are read one at a time).  Loads come from shared memory when the whole team is one CTA
 // that keeps its tables there (S), else through L2 (other CTAs write the
 // records during the launch, so L1 must not serve stale lines).
 template <bool S>
@@ -472,6 +472,11 @@ __device__ __forceinline__ int fold_rows(const StepView& v, int lane, int row, i
     return win;
 }
 
+// Node of a list slot, -1: none.
+__device__ __forceinline__ int slot_node(const BfParams& p, int slot) {
+    return p.slotNode ? __ldg(p.slotNode + slot) : slot < p.n ? slot : -1;
+}
+
 template <class CT, int TK, bool S, int NK>
 __device__ bool relax_slices(const BfParams& p, const StepView& sv, const int* spl, const int* act, int nAct, int s0,
                              int s1, int l, int k) {
@@ -496,7 +501,7 @@ __device__ bool relax_slices(const BfParams& p, const StepView& sv, const int* s
     const int count = all ? s1 - s0 : nAct;
     for (int i = (int)(threadIdx.x >> 5); i < count; i += nwarps) {
         const int s = s0 + (all ? i : act[i]);
-        const int v = __ldg(p.slotNode + s * 32 + lane);
+        const int v = slot_node(p, s * 32 + lane);
         const bool valid = v >= 0;
         const size_t me = cur + (size_t)v * Kp + k;
         double best = (l == 0 && valid) ? ldV<S>(p, me) : kInfD;
@@ -595,11 +600,10 @@ __device__ bool relax_step(const BfParams& p, const Stage& st, int sb, int s0, i
 // overwrites next) has completed it too.  This replaces a grid-wide barrier:
 // a CTA waits only for its graph neighbours.  Returns false, to every thread
 // of the CTA or to none, when a wait ran out of iterations or another CTA
-// raised the error word: one thread reads that word for the CTA (another CTA
-// may raise it between two threads' reads, and the CTA's next barriers need
-// all of it).  The CTA named by
-// p.stallCta (a test hook; -1 in every solve) also waits for a word that no
-// code writes, so its wait runs out.
+// raised the error word: one warp reads that word for the CTA and agrees on it
+// (another CTA may raise it between two threads' reads, and the CTA's next
+// barriers need all of it).  The CTA named by p.stallCta (a test hook; -1 in
+// every solve) also waits for a word that no code writes, so its wait runs out.
 __device__ bool step_handoff(const BfParams& p, const Team& t, unsigned step) {
     __shared__ int sGood;
     __syncthreads();  // the CTA's writes of this step are done
@@ -610,19 +614,21 @@ __device__ bool step_handoff(const BfParams& p, const Team& t, unsigned step) {
         __syncwarp();
         const int w0 = __ldg(p.waitPtr + t.cta), w1 = __ldg(p.waitPtr + t.cta + 1);
         const bool stall = t.cta == p.stallCta;
+        // The error word is read beside each poll, its latency hidden by the
+        // poll's (read after the last one it was 0.2k cycles of every hand-off).
         int good = 1;
-        for (int i0 = w0; i0 < w1 + (stall ? 1 : 0) && good; i0 += 32) {
+        const int wEnd = w1 + (stall ? 1 : 0);
+        for (int i0 = w0; (i0 < wEnd || i0 == w0) && good; i0 += 32) {
             const int i = i0 + (int)threadIdx.x;
             const unsigned* f = i < w1 ? p.stepDone + (size_t)__ldg(p.waitIdx + i) * kStepDoneStride
                                        : (stall && i == w1) ? &p.ctl->neverSet : nullptr;
             unsigned spins = 0;
             for (;;) {
+                const int raised = *(volatile int*)t.err;
                 const bool ready = f == nullptr || (int)(ld_acquire_u32(f) - step) >= 0;
-                if (__all_sync(0xffffffffu, ready)) break;
-                ++spins;
-                if (__any_sync(0xffffffffu, (spins & 63u) == 0 && *(volatile int*)t.err)) { good = 0; break; }
-                if (spins > t.spin) {
-                    if (threadIdx.x == 0) atomicExch(t.err, 1);
+                good = !__any_sync(0xffffffffu, raised != 0);
+                if (__all_sync(0xffffffffu, ready) || !good) break;
+                if (++spins > t.spin) {
                     good = 0;
                     break;
                 }
@@ -631,7 +637,7 @@ __device__ bool step_handoff(const BfParams& p, const Team& t, unsigned step) {
         }
         if (threadIdx.x == 0) {
             if (!good) atomicExch(t.err, 1);
-            sGood = good && *(volatile int*)t.err == 0;
+            sGood = good;
         }
     }
     __syncthreads();
@@ -1798,7 +1804,7 @@ __device__ __forceinline__ bool pair_solve(PairJob& J, BfParams& P, const SolveT
         const CT* c1 = reinterpret_cast<const CT*>(P.cost) + P.layerStride;
         for (long long vv = t.thread(); vv < n; vv += t.nthreads()) {
             const int v = (int)vv;
-            const int slot = __ldg(P.nodeSlot + v), s = slot >> 5, lane = slot & 31;
+            const int slot = P.nodeSlot ? __ldg(P.nodeSlot + v) : v, s = slot >> 5, lane = slot & 31;
             float mean = 0;
             int num = 0;
             for (int j = __ldg(P.spInter + s); j < __ldg(P.spInter + s + 1); ++j) {

@@ -495,7 +495,7 @@ class Graph {
     // the mesh) and keep the template's.
     struct NodeLists {
         LayerTemplate T;
-        DBuf<int> sp[2], src[2], srcDummy, slots, from;
+        DBuf<int> sp[2], src[2], srcDummy, from;
         DBuf<float> f32[2];
         DBuf<double> f64[2];
         bool ready = false;
@@ -1017,9 +1017,6 @@ void Graph::take_node_lists(Run& r) {
             L.src[p].upload(L.T.src[p].data(), L.T.src[p].size(), stream);
         }
         if (T.nY == 2) L.srcDummy.upload(L.T.srcDummy.data(), L.T.srcDummy.size(), stream);
-        std::vector<int> slots((size_t)L.T.nslices * 32, -1);
-        for (int v = 0; v < T.n; ++v) slots[(size_t)v] = v;
-        L.slots.upload(slots.data(), slots.size(), stream);
         const std::vector<int> from = stream_positions(T, L.T);
         L.from.upload(from.data(), from.size(), stream);
         PGC_CUDA(sync_stream());
@@ -1252,8 +1249,8 @@ BfParams Graph::params(const Run& r, int mode, int branchId, double lambda, doub
     const LayerTemplate& L = lists(r);
     const DBuf<int>*sp = r.byNode ? nodeLists.sp : dSp, *src = r.byNode ? nodeLists.src : dSrc;
     const DBuf<int>& dummy = r.byNode ? nodeLists.srcDummy : dSrcDummy;
-    p.slotNode = r.byNode ? nodeLists.slots.p : dSlotNode.p;
-    p.nodeSlot = r.byNode ? nodeLists.slots.p : dNodeSlot.p;
+    p.slotNode = r.byNode ? nullptr : dSlotNode.p;
+    p.nodeSlot = r.byNode ? nullptr : dNodeSlot.p;
     p.spInter = sp[INTER].p;
     p.spIntra = sp[INTRA].p;
     p.srcInter = src[INTER].p;

@@ -45,9 +45,10 @@ def test_a_cta_leaves_a_step_as_one(functions):
     would miss the next barrier."""
     body = functions["step_handoff"]
     assert re.search(r"return sGood != 0;\s*$", body)
-    assert re.search(r"if \(threadIdx\.x == 0\) \{[^{}]*sGood = [^;]*t\.err[^;]*;\s*\}", body)
-    assert "__any_sync(0xffffffffu, (spins & 63u) == 0 && *(volatile int*)t.err)" in body
-    assert body.count("t.err") == body.count("atomicExch(t.err, 1)") + 2
+    assert re.search(r"if \(threadIdx\.x == 0\) \{[^{}]*sGood = good;\s*\}", body)
+    assert "const int raised = *(volatile int*)t.err;" in body
+    assert "good = !__any_sync(0xffffffffu, raised != 0);" in body
+    assert body.count("t.err") == body.count("atomicExch(t.err, 1)") + 1
 
 
 def test_exchanged_records_are_overwritten_after_their_reads(functions):
