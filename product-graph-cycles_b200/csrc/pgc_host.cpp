@@ -412,7 +412,16 @@ class Graph {
     DBuf<unsigned long long> topHist[2];
     bool topHistValid[2] = {false, false};
     EnergyArgs energy_args() const;
-    StreamView stream_view() const {
+    // What only a solve reads -- the in-edge lists, and which of a column's
+    // entries hold an edge -- uploaded for the first one: a handle that exports
+    // its costs pays for none of it.  Without that the list order along the
+    // mesh and the masks cost a new handle's first cost matrix 25 us (162 x 20,
+    // 311 -> 336 us).
+    bool rowMasksReady = false, listsReady = false;
+    void ensure_row_masks();
+    void ensure_lists();
+    StreamView stream_view() {
+        ensure_row_masks();
         return StreamView{T.layerStride(), T.entries[INTER], T.nY, dRowMask.p};
     }
 
@@ -562,20 +571,7 @@ void Graph::upload_template() {
     for (int64_t i = 0; i < 2 * ney; ++i)
         if (EY[(size_t)i] >= nvy) throw Failure(PGC_ERR_ARG, "EY refers to a vertex outside VY");
     cudaStream_t s = stream;
-    for (int p = 0; p < 2; ++p) {
-        dSp[p].upload(T.sp[p].data(), T.sp[p].size(), s);
-        dSrc[p].upload(T.src[p].data(), T.src[p].size(), s);
-        dTedge[p].upload(T.tedge[p].data(), T.tedge[p].size(), s);
-    }
-    dRowMask.alloc((size_t)T.layerStride() / 32);
-    for (int p = 0; p < 2; ++p)
-        PGC_CUDA(launch_row_masks(dTedge[p].p, T.entries[p], dRowMask.p + (p ? T.entries[INTER] / 32 : 0), s));
-    dSlotNode.upload(T.slotNode.data(), T.slotNode.size(), s);
-    dNodeSlot.upload(T.nodeSlot.data(), T.nodeSlot.size(), s);
-    // The closing layer's source list differs from the interlayer one only
-    // with two layers; otherwise the kernels read the interlayer list.
-    if (T.nY == 2) dSrcDummy.upload(T.srcDummy.data(), T.srcDummy.size(), s);
-    else dSrcDummy.release();
+    for (int p = 0; p < 2; ++p) dTedge[p].upload(T.tedge[p].data(), T.tedge[p].size(), s);
     // Template edge endpoints are read on the device only by the SO(3)
     // energies (frames of the edge's source and target).
     if (conj && reg) {
@@ -598,6 +594,29 @@ void Graph::upload_template() {
 }
 
 // Graph-dependent fields of the energy kernels' arguments.
+void Graph::ensure_row_masks() {
+    if (rowMasksReady) return;
+    dRowMask.alloc((size_t)T.layerStride() / 32);
+    for (int p = 0; p < 2; ++p)
+        PGC_CUDA(launch_row_masks(dTedge[p].p, T.entries[p], dRowMask.p + (p ? T.entries[INTER] / 32 : 0), stream));
+    rowMasksReady = true;
+}
+
+void Graph::ensure_lists() {
+    if (listsReady) return;
+    for (int p = 0; p < 2; ++p) {
+        dSp[p].upload(T.sp[p].data(), T.sp[p].size(), stream);
+        dSrc[p].upload(T.src[p].data(), T.src[p].size(), stream);
+    }
+    // The closing layer's source list differs from the interlayer one only
+    // with two layers; otherwise the kernels read the interlayer list.
+    if (T.nY == 2) dSrcDummy.upload(T.srcDummy.data(), T.srcDummy.size(), stream);
+    else dSrcDummy.release();
+    dSlotNode.upload(T.slotNode.data(), T.slotNode.size(), stream);
+    dNodeSlot.upload(T.nodeSlot.data(), T.nodeSlot.size(), stream);
+    listsReady = true;
+}
+
 EnergyArgs Graph::energy_args() const {
     EnergyArgs a{};
     a.n = T.n;
@@ -821,6 +840,7 @@ Graph::Run Graph::prepare_run(int K, bool ratio) {
     if (K < 1) throw Failure(PGC_ERR_ARG, "max depth must be >= 1");
     const long long expanded = (long long)T.n * (T.nY + 1) * K;
     if (expanded >= INT_MAX) throw Failure(PGC_ERR_ARG, "product graph too large for 32-bit expanded node ids");
+    ensure_lists();
     Run r{};
     r.K = K;
     r.Kp = 1;
