@@ -368,6 +368,11 @@ def from_export(directory: str = ".", conjugate: bool = False, regularising_cost
     return g
 
 
+# The Bellman-Ford kernels that a tuned team shape belongs to: raised when they
+# change so that another shape may be the fastest, or one that was may not fit.
+_TEAM_KERNELS = 2  # 1: sweeps in global memory only; 2: local tables
+
+
 def autotune(gen: "product_graph_generator", max_depth: int | None = None, candidates=None,
              cache_path: str | None = None, repeats: int = 2) -> dict:
     """Picks the Bellman-Ford team shape (CTAs, threads per CTA) for the shape
@@ -377,7 +382,8 @@ def autotune(gen: "product_graph_generator", max_depth: int | None = None, candi
     two, layers rounded up to a power of two, max depth, whether layers have
     intralayer edges): a cache file written on one GPU type is not applied
     on another.  A bucket found in the JSON file ``cache_path`` is applied
-    without timing.  Otherwise every candidate (ctas, threads_per_cta) --
+    without timing when it was tuned for the kernels of this library
+    (``_TEAM_KERNELS``; an entry that does not say so was not).  Otherwise every candidate (ctas, threads_per_cta) --
     by default the automatic shape, the automatic CTA count with 320 and 480
     threads, and a half-size team -- is timed over ``repeats`` ratio solves
     (costs regenerated before each; the Bellman-Ford device time of the solve
@@ -399,7 +405,7 @@ def autotune(gen: "product_graph_generator", max_depth: int | None = None, candi
     if cache_path and os.path.exists(cache_path):
         with open(cache_path) as f:
             cache = json.load(f)
-    if key in cache:
+    if cache.get(key, {}).get("kernels") == _TEAM_KERNELS:
         e = cache[key]
         gen.set_team_shape(e["ctas"], e["threads_per_cta"])
         return dict(e, bucket=key, cached=True)
@@ -425,7 +431,7 @@ def autotune(gen: "product_graph_generator", max_depth: int | None = None, candi
                         "team": [int(prof["ctas"]), int(prof["threads"])]})
     best = min(results, key=lambda r: r["bf_ms"])
     entry = {"ctas": best["ctas"], "threads_per_cta": best["threads_per_cta"], "bf_ms": best["bf_ms"],
-             "candidates": results}
+             "candidates": results, "kernels": _TEAM_KERNELS}
     gen.set_team_shape(best["ctas"], best["threads_per_cta"])
     if cache_path:
         # buckets another tuner wrote meanwhile are kept; the file is
