@@ -550,6 +550,12 @@ class Graph {
     void reset_predecessors() {
         PGC_CUDA(cudaMemsetAsync(wPred.p, 0xff, wPred.n * sizeof(int), stream));
     }
+    // Steps of one sweep.  Local tables leave out the closing layer's depths
+    // past the first, which relax nothing.
+    long long sweep_steps(int K, int localKD) const {
+        if (localKD) return (long long)T.nY * localKD;
+        return (long long)(T.nY + 1) * (T.entries[INTRA] == 0 ? 1 : K) - 1;
+    }
     BfParams params(const Run& r, int mode, int branchId, double lambda, double ub);
     Control launch_bf_call(const Run& r, const BfParams& p);
     std::vector<int> read_cycle_buffer(int len);
@@ -1360,7 +1366,7 @@ Control Graph::launch_bf_call(const Run& r, const BfParams& p) {
     stats.cycCand += c.cycCand;
     stats.cycLead += c.cycLead;
     stats.cycStage += c.cycStage;
-    stats.steps += (long long)c.sweeps * ((long long)(T.nY + 1) * (T.entries[INTRA] == 0 ? 1 : r.K) - 1);
+    stats.steps += c.sweeps * sweep_steps(r.K, r.localKD);
     stats.ctas = r.blocks;
     stats.threads = r.threads;
     stats.waitEntries = r.blocks > 1 ? waitEntries : 0;
@@ -1871,7 +1877,7 @@ void Graph::finish_job(const PairJob& J, int K, const Run* r) {
     stats.cycCand = c.cycCand;
     stats.cycLead = c.cycLead;
     stats.cycStage = c.cycStage;
-    stats.steps = J.sweeps * ((long long)(T.nY + 1) * (T.entries[INTRA] == 0 ? 1 : K) - 1);
+    stats.steps = J.sweeps * sweep_steps(K, J.bf.localKD);
     stats.ctas = J.ctas;
     stats.threads = J.threads;
     stats.waitEntries = J.ctas > 1 ? waitEntries : 0;
