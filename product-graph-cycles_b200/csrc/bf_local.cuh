@@ -19,7 +19,7 @@
 // back.  That report does need an order: stepDone is published with release
 // and polled with acquire semantics, a CTA barrier on either side, so that a
 // neighbour's read comes before the store that replaces what it read.  Both are
-// the staging warp's, off the path of the relaxing ones.
+// the staging warp's, once per layer.
 //
 // What it replaces: sources gathered from L2 per in-edge, and a release /
 // acquire hand-off of per-CTA step counters with two CTA barriers around it
@@ -636,15 +636,16 @@ __device__ __noinline__ unsigned local_sweep(int stamp, unsigned step, unsigned 
                 ++step;
                 if (l < nY) {
                     const bool copy = k + 1 < KD ? stage(sb ^ 1, l, k + 1) : stage(sb ^ 1, l + 1, 0);
-                    if (H.ncta > 1) {
-                        // the next step overwrites records published 2 KD - 1
-                        // steps ago; the stall hook's word is one that nothing
-                        // writes
+                    if (H.ncta > 1 && k + 1 == KD) {
+                        // the next layer overwrites the records of the layer
+                        // before this one, which the neighbours have read when
+                        // they have finished that layer; the stall hook's word
+                        // is one that nothing writes
                         const int nWait = H.nWait;
                         for (int i = lane; i < nWait + H.stall; i += 32) {
                             const unsigned* f =
                                 i < nWait ? H.stepDone + (size_t)__ldg(H.waitIdx + i) * kStepDoneStride : H.neverSet;
-                            const int want = i < nWait ? (int)step + 1 - 2 * KD : (int)step;
+                            const int want = i < nWait ? (int)step - KD : (int)step;
                             unsigned spins = 0;
                             while ((int)ld_acquire_u32(f) < want)
                                 if (local_give_up(H, step, spins)) break;
@@ -656,8 +657,10 @@ __device__ __noinline__ unsigned local_sweep(int stamp, unsigned step, unsigned 
                 __syncthreads();
                 // release: the halo reads of the CTA's threads, before the
                 // barrier, come before what the neighbours store after they
-                // have seen this
-                if (lane == 0 && H.ncta > 1) st_release_u32(H.stepDone + (size_t)H.cta * kStepDoneStride, step);
+                // have seen this.  Of the closing layer too: with one depth the
+                // next sweep's first wait is for it.
+                if (lane == 0 && H.ncta > 1 && (k + 1 == KD || l == nY))
+                    st_release_u32(H.stepDone + (size_t)H.cta * kStepDoneStride, step);
                 sb ^= 1;
                 stopped = H.stop[step & 3];
             }
