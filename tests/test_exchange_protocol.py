@@ -45,7 +45,7 @@ def _run(depths, layers, ctas, seed, closing_report=True):
                 continue  # halo records not there yet
             if l < layers and k + 1 == depths and any(done[d] < step - depths for d in near[c]):
                 continue  # a neighbour has not finished the layer before
-            if k + 1 == depths or (closing_report and l == layers):
+            if closing_report if l == layers else k + 1 == depths:
                 done[c] = step
             pos[c] += 1
         idle = 0
