@@ -56,7 +56,7 @@ def test_exchanged_records_are_overwritten_after_their_reads(functions):
     the only order between those reads and the stores that replace the records:
     release and acquire, each beyond a CTA barrier."""
     body = functions["local_sweep"]
-    assert re.search(r"__syncthreads\(\);\s*if \(lane == 0 && [^{}]*\) st_release_u32\(H\.stepDone", body)
+    assert re.search(r"__syncthreads\(\);\s*if \(lane == 0 && [^{}]*\)\s*st_release_u32\(H\.stepDone", body)
     assert "while ((int)ld_acquire_u32(f) < want)" in body
     assert len(re.findall(r"H\.stepDone", body)) == 2
     for f, b in functions.items():
