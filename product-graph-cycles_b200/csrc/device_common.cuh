@@ -304,8 +304,11 @@ constexpr int kTeamWordStride = 8;  // words of a batched-solve team (one sector
 constexpr unsigned kDefaultSpinLimit = 1u << 24;
 // Predecessor loads a literal walk advances per round between team barriers.
 constexpr long long kWalkRoundLoads = 4096;
-// Most threads per Bellman-Ford CTA: 20 warps fit the kernel's registers
-// (about 100 per thread) on one SM without spilling the relaxation loop.
+// Most threads per Bellman-Ford CTA: 20 warps, five to a scheduler, leave 96
+// registers a thread.  The step loop of the sweeps on local tables spills 0-20
+// bytes a thread (24-60 in bf_local_kernel's instances with one depth), the one
+// in global memory 0-40; the set-up and verdict around them up to 0.4 KB, off
+// the step's path.
 constexpr int kBfThreads = 640;
 // Source values a lane gathers before folding them (one batch of rows).
 constexpr int kGather = 20;

@@ -939,9 +939,10 @@ Graph::Run Graph::prepare_run(int K, bool ratio) {
         // Teams on local tables: CTAs of six slices, up to one per SM, and one
         // CTA for up to eight slices.  An exchange costs 1.3k cycles and a
         // slice more on the same schedulers about 0.15k: 162 x 20 (6 slices)
-        // takes 0.56 ms with one CTA and 0.72 with two, 642 x 60 (21 slices)
-        // 1.08 with one and 2, 1.02 with four, 1.10 with eleven, 1,777 x 97 (56)
-        // 5.3 ms with CTAs of four slices, 4.5 of six, 4.6 of eight, 5.4 of 19.
+        // takes 0.54 ms with one CTA and 0.72 with two, 642 x 60 (21 slices)
+        // 1.16 with one, 1.05 with two, 1.01 with four, 1.11 with eleven,
+        // 1,777 x 97 (56) 5.3 ms with CTAs of four slices, 4.4 of six, 4.6 of
+        // eight, 5.4 of 19.
         int active = 0;
         for (int s = 0; s < T.nslices; ++s)
             if (T.sp[INTER][(size_t)s + 1] > T.sp[INTER][(size_t)s]) ++active;
