@@ -540,15 +540,15 @@ __device__ __forceinline__ double4 ldg_quat(const double4* q) {
 }
 
 // Work item: a block of template positions x a chunk of layers.  A thread
-// keeps two positions, the same lane of two consecutive rows -- template edge,
-// Y pattern, X columns, frames, the X half of the line integral -- and walks
-// the chunk's layers, so per layer it reads only the layer's Y edge, the fd
-// entry and the frames; the stores of a warp stay 32 consecutive entries of
-// one layer.  In-edges come in pairs that leave the same X edge (a node and
-// its degenerate copy), so the two rows often join the same two frames: their
-// distance and its robust loss, an arc cosine and two powers, are then
-// computed once (and the fd entry, of the same target, read once).  Every
-// value is computed with the same operations in the same order as per entry.
+// keeps ROWS positions, the same lane of consecutive rows -- template edge, Y
+// pattern, X columns, frames, the X half of the line integral -- and walks the
+// chunk's layers, so per layer it reads only the layer's Y edge, the fd entry
+// and the frames; the stores of a warp stay 32 consecutive entries of one
+// layer.  A pruned graph's in-edges come in pairs that leave the same X edge (a
+// node and its degenerate copy), so two rows often join the same two frames:
+// their distance and its robust loss, an arc cosine and two powers, are then
+// computed once (and the fd entry, of the same target, read once).  Every value
+// is computed with the same operations in the same order as per entry.
 constexpr int kHoLayerChunk = 16;
 
 struct HoPosition {
@@ -558,6 +558,7 @@ struct HoPosition {
     double dxx[3];
 };
 
+template <int ROWS>
 __global__ void __launch_bounds__(256) ho_energy_kernel(EnergyArgs a) {
     extern __shared__ unsigned int topSh[];  // [2][kTopBins] when a.hist0
     DigitRun r0, r1;
@@ -570,19 +571,19 @@ __global__ void __launch_bounds__(256) ho_energy_kernel(EnergyArgs a) {
     // same number for every edge, computed once per thread by the same code.
     const double rl0 = robust_loss(a, 0.0);
     const int stride = (int)a.layerStride, inter = (int)a.interEntries, layers = a.nY + 1;
-    const int perBlock = 2 * (int)blockDim.x;
+    const int perBlock = ROWS * (int)blockDim.x;
     const int posBlocks = (stride + perBlock - 1) / perBlock;
     const int chunks = (layers + kHoLayerChunk - 1) / kHoLayerChunk;
     const long long items = (long long)posBlocks * chunks;
     for (long long it = blockIdx.x; it < items; it += gridDim.x) {
         const int lc = (int)(it / posBlocks);
-        const int pos0 = (int)(it - (long long)lc * posBlocks) * perBlock + (int)(threadIdx.x >> 5) * 64 +
+        const int pos0 = (int)(it - (long long)lc * posBlocks) * perBlock + (int)(threadIdx.x >> 5) * 32 * ROWS +
                          (int)(threadIdx.x & 31);
         if (pos0 >= stride) continue;
         const int l0 = lc * kHoLayerChunk, l1 = min(l0 + kHoLayerChunk, layers);
-        HoPosition P[2];
+        HoPosition P[ROWS];
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
+        for (int u = 0; u < ROWS; ++u) {
             HoPosition& q = P[u];
             const int pos = pos0 + 32 * u;
             q.isInter = pos < inter;
@@ -612,15 +613,18 @@ __global__ void __launch_bounds__(256) ho_energy_kernel(EnergyArgs a) {
                 q.trgtNext = __ldg(a.eNext + t);
             }
         }
-        const bool both = P[0].on && P[1].on && P[0].isInter == P[1].isInter;
-        const bool sameFrames = both && a.quat && P[0].src == P[1].src && P[0].srcBack == P[1].srcBack &&
-                                P[0].trgt == P[1].trgt && P[0].trgtBack == P[1].trgtBack &&
-                                P[0].trgtNext == P[1].trgtNext;
-        const bool sameFd = both && P[0].x2 == P[1].x2 && P[0].pat == P[1].pat;
+        bool sameFrames = false, sameFd = false;
+        if constexpr (ROWS == 2) {
+            const HoPosition &p = P[0], &q = P[1];
+            const bool both = p.on && q.on && p.isInter == q.isInter;
+            sameFrames = both && a.quat && p.src == q.src && p.srcBack == q.srcBack && p.trgt == q.trgt &&
+                         p.trgtBack == q.trgtBack && p.trgtNext == q.trgtNext;
+            sameFd = both && p.x2 == q.x2 && p.pat == q.pat;
+        }
         for (int l = l0; l < l1; ++l) {
             double so3 = 0.0, rl = rl0, fd = 0.0;
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
+            for (int u = 0; u < ROWS; ++u) {
                 const HoPosition& q = P[u];
                 const int pos = pos0 + 32 * u;
                 if (pos >= stride) break;
@@ -1530,10 +1534,22 @@ cudaError_t launch_plain_energy(const EnergyArgs& a, cudaStream_t s, bool shared
     plain_energy_kernel<<<stream_grid(plain_energy_kernel, 256, smem, shared ? a.total : -1), 256, smem, s>>>(a, chunk);
     return cudaGetLastError();
 }
+// Rows a thread takes.  Two where rows come in pairs that join the same frames
+// -- a pruned graph's, with frames -- and there is a two-row work item for
+// every SM: pruned 600 x 30 57 us (one row 63), 1,000 x 40 89 (106), 5,000 x
+// 100 0.92 ms (1.21), but 300 x 20 48 us (42).  One elsewhere: the second row shares next to
+// nothing and halves the warps (unpruned 5,000 x 200 without frames 1.32 ms,
+// two rows 1.70; with frames 5.4 and 6.1; 300 x 20 52 us and 76).
+static int ho_rows(const EnergyArgs& a) {
+    if (!a.quat || !a.quatPrune) return 1;
+    const long long items = ((a.layerStride + 511) / 512) * ((a.nY + kHoLayerChunk) / kHoLayerChunk);
+    return items >= 148 ? 2 : 1;
+}
 cudaError_t launch_ho_energy(const EnergyArgs& a, cudaStream_t s) {
     const size_t smem = a.hist0 ? 2 * kTopBins * sizeof(unsigned) : 0;
     note_launch();
-    ho_energy_kernel<<<stream_grid(ho_energy_kernel, 256, smem), 256, smem, s>>>(a);
+    if (ho_rows(a) == 2) ho_energy_kernel<2><<<stream_grid(ho_energy_kernel<2>, 256, smem), 256, smem, s>>>(a);
+    else ho_energy_kernel<1><<<stream_grid(ho_energy_kernel<1>, 256, smem), 256, smem, s>>>(a);
     return cudaGetLastError();
 }
 // part: kFdMaxBlocks + 1 entries, the last one the result.
