@@ -1529,8 +1529,11 @@ cudaError_t launch_plain_energy(const EnergyArgs& a, cudaStream_t s, bool shared
     const size_t smem = a.hist0 ? 2 * kTopBins * sizeof(unsigned) : 0;
     note_launch();
     // sixteen layers a thread, fewer where that would leave SMs idle: a wave of
-    // four blocks per SM takes chunks of four layers up to 2.4 M entries
-    const int chunk = a.total < 148LL * 4 * 256 * 16 ? 4 : 16;
+    // four blocks per SM takes chunks of four layers up to 2.4 M entries, and
+    // of two below one entry a thread (162 x 20 with the line integral 6.1 us,
+    // chunks of four 7.3; 162 x 100 9.5 and 9.0)
+    const long long wave = 148LL * 4 * 256;
+    const int chunk = a.total < wave ? 2 : a.total < 16 * wave ? 4 : 16;
     plain_energy_kernel<<<stream_grid(plain_energy_kernel, 256, smem, shared ? a.total : -1), 256, smem, s>>>(a, chunk);
     return cudaGetLastError();
 }
